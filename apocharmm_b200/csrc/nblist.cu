@@ -666,6 +666,13 @@ void NeighborList::alloc() {
   APO_CUDA(cudaMemset(xyzq_s, 0, (size_t)S * sizeof(float4)));
   APO_CUDA(cudaMemset(perm, 0xff, (size_t)S * sizeof(int)));
   APO_CUDA(cudaMemset(type_s, 0, (size_t)S * sizeof(int)));
+  // until the first build an atom's slot is slot 0 and a cluster's column
+  // column 0: an integrator given a context before any list exists projects
+  // the positions onto the constraints first (and writes through glo2loc),
+  // and a build whose column overflowed leaves that column's clusters as
+  // they were; both must index inside the arrays
+  APO_CUDA(cudaMemset(glo2loc, 0, (size_t)n * sizeof(int)));
+  APO_CUDA(cudaMemset(m_cl_col, 0, (size_t)ncl * sizeof(int)));
 }
 
 void NeighborList::build(const float4 *d_xyzq, cudaStream_t s) {

@@ -333,3 +333,33 @@ def test_settings_changed_between_calls_take_effect(tmp_path):
     t600 = ctx.computeTemperature()
     assert 200.0 < t300 < 450.0
     assert t600 > 480.0, (t300, t600)
+
+
+@pytest.mark.parametrize("kind", ["langevin", "nose_hoover", "piston"])
+def test_context_without_a_list_is_accepted(tmp_path, kind):
+    """Coordinates set from an array, then straight to the integrator: no list
+    exists yet when the positions are projected onto the constraints (every
+    slot index must be valid all the same), and the run is the one that an
+    evaluation beforehand gives."""
+    out = []
+    for rep in range(2):
+        s = water_box(1000, 31.0, seed=3)
+        keep = api.system_context(s, str(tmp_path / f"r{rep}"), settings=SMALL)
+        ctx = keep[3]
+        if rep == 1:
+            ctx.calculateForces(False, False, False)
+        it = {"langevin": api.CudaLangevinThermostatIntegrator,
+              "nose_hoover": api.CudaNoseHooverIntegrator,
+              "piston": api.CudaLangevinPistonIntegrator}[kind](0.0001)
+        if kind == "langevin":
+            it.setThermostatRngSeed(5)
+        if kind == "piston":
+            it.setCrystalType(it.CUBIC)
+            it.setLangevinPistonFrictionSeed(5)
+        it.setCharmmContext(ctx)
+        it.propagate(2)
+        out.append(ctx.getCoordinates())
+    # the two lists are built from positions a projection apart, so single-
+    # precision sums differ by their rounding: 1e-6 of a contact's gradient of
+    # up to 1e5 kcal/mol/A moves a hydrogen by dt^2 g / m = 4e-7 A in 0.1 fs
+    assert np.abs(out[0] - out[1]).max() < 1e-6
