@@ -32,6 +32,7 @@ struct Scalars {
   long long window;
   unsigned counter;
   unsigned pad;
+  double pc_a, pc_b;         // Nose-Hoover: displacement = pc_a delta + pc_b delta_prev
 };
 
 struct SettleConst {
@@ -213,6 +214,87 @@ __device__ void sum_partials(const double *partials, double &s0, double &s1) {
   s1 = b;
 }
 
+// Sums of N values (N <= 32) over the lanes of a warp by halving exchanges:
+// at every level a lane hands half of its values over and adds the half it
+// gets, so N = 32 takes 31 exchanges instead of 160.  On return lane L holds
+// the total of value slot_of_lane<P>(L) in v[0], P the next power of two.
+template <int N>
+struct Pow2 {
+  static constexpr int value = N <= 1 ? 1 : N <= 2 ? 2 : N <= 4 ? 4 : N <= 8 ? 8 : N <= 16 ? 16 : 32;
+};
+template <int P>
+__device__ __forceinline__ void warp_sum_scatter(double (&v)[P]) {
+  const int lane = threadIdx.x & 31;
+  int o = 16;
+#pragma unroll
+  for (int half = P / 2; half >= 1; half >>= 1, o >>= 1) {
+    const bool hi = lane & o;
+#pragma unroll
+    for (int i = 0; i < half; ++i) {
+      const double send = hi ? v[i] : v[i + half];
+      const double keep = hi ? v[i + half] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+}
+// the value whose total a lane holds, and whether it is the lane that
+// publishes it
+template <int P>
+__device__ __forceinline__ int slot_of_lane() {
+  return (threadIdx.x & 31) / (32 / P);
+}
+template <int P>
+__device__ __forceinline__ bool publishes() {
+  return (threadIdx.x & 31) % (32 / P) == 0;
+}
+
+// block-wide sums of N values; partials[N * block + k]
+template <int N>
+__device__ void block_partials_n(const double (&in)[N], double *partials) {
+  constexpr int P = Pow2<N>::value;
+  __shared__ double sh[N][kThreads / 32];
+  double v[P];
+#pragma unroll
+  for (int k = 0; k < P; ++k) v[k] = k < N ? in[k] : 0.0;
+  warp_sum_scatter<P>(v);
+  if (publishes<P>() && slot_of_lane<P>() < N) sh[slot_of_lane<P>()][threadIdx.x >> 5] = v[0];
+  __syncthreads();
+  if (threadIdx.x < N) {
+    double s = 0;
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w) s += sh[threadIdx.x][w];
+    partials[N * blockIdx.x + threadIdx.x] = s;
+  }
+}
+
+// totals of the N partials of every block into tot[] (shared memory), in an
+// order fixed by the grid: thread t takes blocks t, t + 128, ...; all of a
+// block's values are loaded together, so the last block waits for a few
+// memory latencies instead of one per block of the grid
+template <int N>
+__device__ void sum_partials_n(const double *partials, double *tot) {
+  constexpr int P = Pow2<N>::value;
+  __shared__ double sh[N][kThreads / 32];
+  double v[P];
+#pragma unroll
+  for (int k = 0; k < P; ++k) v[k] = 0.0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += kThreads) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] += partials[(size_t)N * b + k];
+  }
+  warp_sum_scatter<P>(v);
+  if (publishes<P>() && slot_of_lane<P>() < N) sh[slot_of_lane<P>()][threadIdx.x >> 5] = v[0];
+  __syncthreads();
+  if (threadIdx.x < N) {
+    double s = 0;
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w) s += sh[threadIdx.x][w];
+    tot[threadIdx.x] = s;
+  }
+  __syncthreads();
+}
+
 struct Common {
   // several systems: atom -> system, first atom of every system, and every
   // system's noise seed (null for one system)
@@ -228,7 +310,7 @@ struct Common {
   const int4 *groups;   // atoms (-1 unused)
   const int2 *gmeta;    // (kind, shake parameter index)
   const float4 *shake_p;
-  double4 *coords, *vel, *dprev, *delta, *dpred, *ref;
+  double4 *coords, *vel, *dprev, *delta;
   float4 *xyzq;
   long long *force;
   int stride;
@@ -389,197 +471,242 @@ __global__ void __launch_bounds__(kThreads) langevin_kernel(Common c, double gam
   }
 }
 
+// ------------------------------------------------- groups on W lanes each
+// The Nose-Hoover and piston kernels handle a constraint group of up to four
+// atoms on W = 4 lanes (an atom each; positions exchanged by shuffles and the
+// constraint worked out in every lane, as the Langevin kernel does) or on
+// W = 1 (one thread loops over the atoms).  Four lanes hide the latency of the
+// dependent loads when the groups alone do not fill the GPU; one lane does a
+// quarter of the FP64 constraint arithmetic, which is what counts once they
+// do.
+// (35,000 groups: the same within the spread, 15.9 ms for 40 Nose-Hoover steps
+// of 107,000 atoms either way; 333,000 groups: one lane is 2 % faster, 59.1
+// against 60.3 ms for 20 steps of 998,000 atoms)
+constexpr int kFourLaneGroups = 65536;
+template <int W>
+struct GroupLane {
+  static constexpr int K = 4 / W;  // atoms of this thread
+  int at[K];
+  bool on[K];
+  int m = 0;         // atoms of the group
+  int2 meta;
+  bool valid;
+  __device__ __forceinline__ explicit GroupLane(const Common &c) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int g = t / W;
+    valid = g < c.ngroups;
+    meta = make_int2(0, 0);
+    int all[4] = {0, 0, 0, 0};
+    if (valid) {
+      m = group_atoms(c, g, all);
+      meta = c.gmeta[g];
+    }
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const int k = W == 1 ? j : (t & 3);
+      on[j] = valid && k < m;
+      at[j] = W == 1 ? all[j] : (k == 0 ? all[0] : k == 1 ? all[1] : k == 2 ? all[2] : all[3]);
+    }
+  }
+  // n moved onto the group's constraints with o as the constrained reference
+  __device__ __forceinline__ void constrain(const Common &c, const d3 (&o)[K], d3 (&n)[K]) const {
+    if constexpr (W == 1) {
+      if (valid) apply_constraint(meta.x, m, o, n, c.sk, c.shake_p, meta.y);
+    } else {
+      const int base = (threadIdx.x & 31) & ~3;
+      d3 og[4], ng[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        og[q] = mk(__shfl_sync(0xffffffffu, o[0].x, base + q),
+                   __shfl_sync(0xffffffffu, o[0].y, base + q),
+                   __shfl_sync(0xffffffffu, o[0].z, base + q));
+        ng[q] = mk(__shfl_sync(0xffffffffu, n[0].x, base + q),
+                   __shfl_sync(0xffffffffu, n[0].y, base + q),
+                   __shfl_sync(0xffffffffu, n[0].z, base + q));
+      }
+      if (valid) apply_constraint(meta.x, m, og, ng, c.sk, c.shake_p, meta.y);
+      n[0] = pick(ng, threadIdx.x & 3);
+    }
+  }
+};
+
 // -------------------------------------------------------- Nose-Hoover step
-// src/CudaNoseHooverIntegrator.cu:647-1004, split at the grid-wide
-// kinetic-energy reductions:
-//   K0 half step + constraint + KE(v_old) + piston update
-//   K1..K3 predictor-corrector (K1, K2 also KE + piston)
-//   K4 constraint + on-step velocity + KE + piston + average temperature
+// src/CudaNoseHooverIntegrator.cu:647-1004 in two launches.  Its three
+// predictor-corrector passes
+//   v <- (delta_prev + d) / (2 dt),  d <- delta - dt^2 xi v   (d = delta at first)
+// are linear in the two displacements of an atom, d = a delta + b delta_prev
+// with the same a and b for every atom, and the kinetic energy that moves the
+// piston between them is a quadratic form in a and b with the three sums
+// over m delta_prev^2, m delta_prev delta and m delta^2 as coefficients.  So
+// the passes are scalar arithmetic in the last block of the half step (no
+// pass over the atoms), and the final kernel forms a delta + b delta_prev
+// itself.  The same numbers up to the rounding of FP64 sums; an atom moves
+// 470 bytes a step instead of about 1,300.  Bound by memory at a million atoms
+// (20 steps of 998,000 atoms: 71.0 -> 66.7 ms) and by latency below (40 steps
+// of 107,000 atoms: 21.3 -> 20.4 ms).
 __device__ void piston_update(Scalars *sc, double ke_sel, double ke_ref, double dt) {
   sc->piston_f = 2.0 * dt * (ke_sel - ke_ref) / sc->piston_mass;
   if (sc->piston_f_prev == 0.0) sc->piston_f_prev = sc->piston_f;
   sc->piston_v = sc->piston_v_prev + 0.5 * (sc->piston_f + sc->piston_f_prev);
 }
 
+template <int W>
 __global__ void __launch_bounds__(kThreads) nh_half_kernel(Common c, double ke_ref, int use_old) {
-  if (*c.err) return;
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr int K = 4 / W;
+  const unsigned err = *c.err;  // looked at before the first store, with the loads under way
   const double dt = c.dt, dt2 = dt * dt, idt = 1.0 / dt;
-  double ke0 = 0, ke1 = 0;
-  if (g < c.ngroups) {
-    int at[4];
-    const int m = group_atoms(c, g, at);
-    const int2 meta = c.gmeta[g];
-    // every load of the group first (each level of the chain atom -> slot ->
-    // gradient for all atoms at once), then the arithmetic, then the stores:
-    // at a million atoms the kernel is bound by memory latency
-    double4 x[4], vm[4], dp[4];
-    int slot[4];
+  const GroupLane<W> G(c);
+  // every load of the thread first, each level of the chain atom -> slot ->
+  // gradient for all its atoms at once
+  double4 x[K], vm[K], dp[K];
+  int slot[K];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (k < m) {
-        const int a = at[k];
-        x[k] = c.coords[a];
-        vm[k] = c.vel[a];
-        dp[k] = c.dprev[a];
-        slot[k] = c.glo2loc[a];
-      }
-    }
-    long long gi[4][3];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (k < m) {
-        gi[k][0] = c.force[slot[k]];
-        gi[k][1] = c.force[c.stride + slot[k]];
-        gi[k][2] = c.force[2 * c.stride + slot[k]];
-      }
-    }
-    d3 o[4], n[4], n0[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (k < m) {  // the slots are cleared for the next force evaluation
-        c.force[slot[k]] = 0;
-        c.force[c.stride + slot[k]] = 0;
-        c.force[2 * c.stride + slot[k]] = 0;
-        const d3 gr = mk((double)gi[k][0] * kInvForceScale, (double)gi[k][1] * kInvForceScale,
-                         (double)gi[k][2] * kInvForceScale);
-        o[k] = xyz(x[k]);
-        n[k] = o[k] + (xyz(dp[k]) - (dt2 * vm[k].w) * gr);
-        n0[k] = n[k];
-      }
-    }
-    apply_constraint(meta.x, m, o, n, c.sk, c.shake_p, meta.y);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (k < m) {
-        const int a = at[k];
-        const d3 d = n[k] - o[k];
-        c.ref[a] = x[k];
-        c.delta[a] = make_double4(d.x, d.y, d.z, 0.0);
-        c.dpred[a] = make_double4(d.x, d.y, d.z, 0.0);
-        c.coords[a] = make_double4(n[k].x, n[k].y, n[k].z, x[k].w);
-        const double mass = 1.0 / vm[k].w;
-        // the on-step velocity of the first predictor-corrector pass carries
-        // the constraint's displacement over dt, as the reference's constraint
-        // pass adds it to the velocities (src/CudaHolonomicConstraint.cu:94-106,
-        // src/CudaNoseHooverIntegrator.cu:905-930)
-        const d3 v = xyz(vm[k]) + idt * (n[k] - n0[k]);
-        const d3 u1 = idt * xyz(dp[k]), u2 = idt * d;
-        const double kon = 0.5 * mass * dot(v, v);
-        ke0 += (0.5 * mass * dot(u1, u1) + kon + 0.5 * mass * dot(u2, u2)) / 3.0;
-        ke1 += kon;
-      }
+  for (int j = 0; j < K; ++j) {
+    x[j] = vm[j] = dp[j] = make_double4(0.0, 0.0, 0.0, 0.0);
+    slot[j] = 0;
+    if (G.on[j]) {
+      const int a = G.at[j];
+      x[j] = c.coords[a];
+      vm[j] = c.vel[a];
+      dp[j] = c.dprev[a];
+      slot[j] = c.glo2loc[a];
     }
   }
-  block_partials(ke0, ke1, c.partials);
+  long long gi[K][3];
+#pragma unroll
+  for (int j = 0; j < K; ++j) {
+    if (G.on[j]) {
+      gi[j][0] = c.force[slot[j]];
+      gi[j][1] = c.force[c.stride + slot[j]];
+      gi[j][2] = c.force[2 * c.stride + slot[j]];
+    }
+  }
+  if (err) return;
+  d3 o[K], n[K], n0[K];
+#pragma unroll
+  for (int j = 0; j < K; ++j) {
+    o[j] = xyz(x[j]);
+    n[j] = o[j];
+    if (G.on[j]) {  // the slots are cleared for the next force evaluation
+      c.force[slot[j]] = 0;
+      c.force[c.stride + slot[j]] = 0;
+      c.force[2 * c.stride + slot[j]] = 0;
+      const d3 gr = mk((double)gi[j][0] * kInvForceScale, (double)gi[j][1] * kInvForceScale,
+                       (double)gi[j][2] * kInvForceScale);
+      n[j] = o[j] + (xyz(dp[j]) - (dt2 * vm[j].w) * gr);
+    }
+    n0[j] = n[j];
+  }
+  G.constrain(c, o, n);
+  // [0] twice the on-step kinetic energy, [1] sum m delta_prev^2,
+  // [2] sum m delta_prev delta, [3] sum m delta^2
+  double v[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int j = 0; j < K; ++j) {
+    if (G.on[j]) {
+      const d3 d = n[j] - o[j], p = xyz(dp[j]);
+      c.delta[G.at[j]] = make_double4(d.x, d.y, d.z, 0.0);
+      const double mass = 1.0 / vm[j].w;
+      // the on-step velocity of the first predictor-corrector pass carries
+      // the constraint's displacement over dt, as the reference's constraint
+      // pass adds it to the velocities (src/CudaHolonomicConstraint.cu:94-106,
+      // src/CudaNoseHooverIntegrator.cu:905-930)
+      const d3 u = xyz(vm[j]) + idt * (n[j] - n0[j]);
+      v[0] += mass * dot(u, u);
+      v[1] += mass * dot(p, p);
+      v[2] += mass * dot(p, d);
+      v[3] += mass * dot(d, d);
+    }
+  }
+  block_partials_n<4>(v, c.partials);
   if (is_last_block(&c.sc->counter)) {
-    double s0, s1;
-    sum_partials(c.partials, s0, s1);
+    __shared__ double tot[4];
+    sum_partials_n<4>(c.partials, tot);
     if (threadIdx.x == 0) {
-      c.sc->piston_v_prev = c.sc->piston_v;
-      c.sc->piston_f_prev = c.sc->piston_f;
-      piston_update(c.sc, use_old ? s1 : s0, ke_ref, dt);
-      c.sc->counter = 0;
-    }
-  }
-}
-
-// predictor-corrector pass over atoms; with KE also the next piston update
-template <bool KE>
-__global__ void __launch_bounds__(kThreads) nh_pc_kernel(Common c, int natom, double ke_ref,
-                                                         int use_old) {
-  if (*c.err) return;
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  const double dt = c.dt, idt = 1.0 / dt, fact = 0.5 / dt;
-  const double xi = c.sc->piston_v;
-  double ke0 = 0, ke1 = 0;
-  if (a < natom) {
-    const d3 dprev = xyz(c.dprev[a]), dpred = xyz(c.dpred[a]), d = xyz(c.delta[a]);
-    const d3 v = fact * (dprev + dpred);
-    const d3 np = d - (dt * dt * xi) * v;
-    c.dpred[a] = make_double4(np.x, np.y, np.z, 0.0);
-    c.vel[a] = make_double4(v.x, v.y, v.z, c.vel[a].w);
-    const d3 r = xyz(c.ref[a]);
-    c.coords[a] = make_double4(r.x + np.x, r.y + np.y, r.z + np.z, c.coords[a].w);
-    if (KE) {
-      const double mass = 1.0 / c.vel[a].w;
-      const d3 u1 = idt * dprev, u2 = idt * d;
-      const double kon = 0.5 * mass * dot(v, v);
-      ke0 = (0.5 * mass * dot(u1, u1) + kon + 0.5 * mass * dot(u2, u2)) / 3.0;
-      ke1 = kon;
-    }
-  }
-  if (KE) {
-    block_partials(ke0, ke1, c.partials);
-    if (is_last_block(&c.sc->counter)) {
-      double s0, s1;
-      sum_partials(c.partials, s0, s1);
-      if (threadIdx.x == 0) {
-        piston_update(c.sc, use_old ? s1 : s0, ke_ref, dt);
-        c.sc->counter = 0;
+      Scalars *sc = c.sc;
+      sc->piston_v_prev = sc->piston_v;
+      sc->piston_f_prev = sc->piston_f;
+      // the half-step energies of both sides, 1/2 m u^2 with u over dt
+      const double half = 0.5 * idt * idt * (tot[1] + tot[3]), fact = 0.5 * idt;
+      double kon = 0.5 * tot[0];
+      double pa = 1.0, pb = 0.0;
+      for (int pass = 0; pass < 3; ++pass) {
+        piston_update(sc, use_old ? kon : (half + kon) / 3.0, ke_ref, dt);
+        const double qa = pa, qb = 1.0 + pb;  // v = fact (qa delta + qb delta_prev)
+        kon = 0.5 * fact * fact *
+              (qb * qb * tot[1] + 2.0 * qa * qb * tot[2] + qa * qa * tot[3]);
+        const double f = dt2 * sc->piston_v * fact;
+        pa = 1.0 - f * qa;
+        pb = -f * qb;
       }
+      sc->pc_a = pa;
+      sc->pc_b = pb;
+      sc->counter = 0;
     }
   }
 }
 
+template <int W>
 __global__ void __launch_bounds__(kThreads) nh_final_kernel(Common c, double ke_ref, int use_old) {
-  if (*c.err) return;
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr int K = 4 / W;
+  const unsigned err = *c.err;
   const double dt = c.dt, idt = 1.0 / dt, fact = 0.5 / dt;
-  double ke0 = 0, ke1 = 0;
-  if (g < c.ngroups) {
-    int at[4];
-    const int m = group_atoms(c, g, at);
-    const int2 meta = c.gmeta[g];
-    // loads first (as nh_half_kernel), then the constraint, then the stores
-    d3 o[4], n[4], dp[4];
-    double q[4], im[4];
-    int slot[4];
+  const double pa = c.sc->pc_a, pb = c.sc->pc_b;
+  const GroupLane<W> G(c);
+  d3 o[K], n[K], dp[K];
+  double q[K], im[K];
+  int slot[K];
+  double4 so[K];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (k < m) {
-        const int a = at[k];
-        o[k] = xyz(c.ref[a]);
-        const double4 x = c.coords[a];
-        n[k] = xyz(x);
-        q[k] = x.w;
-        dp[k] = xyz(c.dprev[a]);
-        im[k] = c.vel[a].w;
-        slot[k] = c.glo2loc[a];
-      }
-    }
-    double4 so[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-      if (k < m) so[k] = c.slot_off[slot[k]];
-    apply_constraint(meta.x, m, o, n, c.sk, c.shake_p, meta.y);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (k < m) {
-        const int a = at[k];
-        const d3 d = n[k] - o[k];
-        const d3 v = fact * (d + dp[k]);
-        const double mass = 1.0 / im[k];
-        const d3 u1 = idt * dp[k], u2 = idt * d;
-        const double kon = 0.5 * mass * dot(v, v);
-        ke0 += (0.5 * mass * dot(u1, u1) + kon + 0.5 * mass * dot(u2, u2)) / 3.0;
-        ke1 += kon;
-        c.vel[a] = make_double4(v.x, v.y, v.z, im[k]);
-        c.dprev[a] = make_double4(d.x, d.y, d.z, 0.0);
-        c.coords[a] = make_double4(n[k].x, n[k].y, n[k].z, q[k]);
-        c.xyzq[a] = make_float4((float)n[k].x, (float)n[k].y, (float)n[k].z, (float)q[k]);
-        c.xyzq_s[slot[k]] = make_float4((float)(n[k].x + so[k].x), (float)(n[k].y + so[k].y),
-                                        (float)(n[k].z + so[k].z), (float)q[k]);
-      }
+  for (int j = 0; j < K; ++j) {
+    o[j] = n[j] = dp[j] = mk(0.0, 0.0, 0.0);
+    q[j] = im[j] = 0.0;
+    slot[j] = 0;
+    if (G.on[j]) {
+      const int a = G.at[j];
+      const double4 x = c.coords[a];
+      o[j] = xyz(x);
+      q[j] = x.w;
+      dp[j] = xyz(c.dprev[a]);
+      n[j] = xyz(c.delta[a]);
+      im[j] = c.vel[a].w;
+      slot[j] = c.glo2loc[a];
     }
   }
-  block_partials(ke0, ke1, c.partials);
+#pragma unroll
+  for (int j = 0; j < K; ++j) {
+    if (G.on[j]) so[j] = c.slot_off[slot[j]];
+    n[j] = o[j] + (pa * n[j] + pb * dp[j]);
+  }
+  if (err) return;
+  G.constrain(c, o, n);
+  double v[2] = {0.0, 0.0};
+#pragma unroll
+  for (int j = 0; j < K; ++j) {
+    if (G.on[j]) {
+      const int a = G.at[j];
+      const d3 d = n[j] - o[j];
+      const d3 u = fact * (d + dp[j]);
+      const double mass = 1.0 / im[j];
+      const d3 u1 = idt * dp[j], u2 = idt * d;
+      const double kon = 0.5 * mass * dot(u, u);
+      v[0] += (0.5 * mass * dot(u1, u1) + kon + 0.5 * mass * dot(u2, u2)) / 3.0;
+      v[1] += kon;
+      c.vel[a] = make_double4(u.x, u.y, u.z, im[j]);
+      c.dprev[a] = make_double4(d.x, d.y, d.z, 0.0);
+      c.coords[a] = make_double4(n[j].x, n[j].y, n[j].z, q[j]);
+      c.xyzq[a] = make_float4((float)n[j].x, (float)n[j].y, (float)n[j].z, (float)q[j]);
+      c.xyzq_s[slot[j]] = make_float4((float)(n[j].x + so[j].x), (float)(n[j].y + so[j].y),
+                                      (float)(n[j].z + so[j].z), (float)q[j]);
+    }
+  }
+  block_partials_n<2>(v, c.partials);
   if (is_last_block(&c.sc->counter)) {
-    double s0, s1;
-    sum_partials(c.partials, s0, s1);
+    __shared__ double tot[2];
+    sum_partials_n<2>(c.partials, tot);
     if (threadIdx.x == 0) {
-      piston_update(c.sc, use_old ? s1 : s0, ke_ref, dt);
-      finish_temperature(c, s0, s1);
+      piston_update(c.sc, use_old ? tot[1] : tot[0], ke_ref, dt);
+      finish_temperature(c, tot[0], tot[1]);
       c.sc->step += 1;
       c.sc->counter = 0;
     }
@@ -716,16 +843,24 @@ __global__ void com_apply_kernel(Common c, int natom, int freq) {
 }
 
 // --------------------------------------------------------- Langevin piston
-// src/CudaLangevinPistonIntegrator.cu:1705-2060 in three kinds of launch:
-//   lp_half   half step, constraint, constraint forces and virial, the
-//             pressure tensor and its static part; last block: the first
-//             pass's piston move (one normal per piston degree of freedom)
-//             and thermostat update from its kinetic energy
-//   lp_pc     (per pass) atoms follow piston and thermostat; last block:
-//             the pressure difference with the new half-step kinetic term,
-//             then the next pass's piston move and thermostat update
-//   lp_final  constraints on the new and the scaled reference positions,
-//             on-step velocities, kinetic energy, pressure averages, the box
+// src/CudaLangevinPistonIntegrator.cu:1705-2060 in two launches (and one for
+// the list's shifts):
+//   lp_half   half step, constraint, constraint forces and virial, the sums
+//             that the pressure and the kinetic energies are made of; last
+//             block: the pressure tensor and its static part, then every
+//             predictor-corrector pass (piston move with one normal per
+//             piston degree of freedom, thermostat update, the pass's
+//             displacements, pressure difference and kinetic energy) as
+//             scalar arithmetic: a pass is linear in an atom's two
+//             displacements with the same factors for every atom
+//   lp_final  the last pass's positions and displacements, constraints on
+//             the new and the scaled reference positions, on-step
+//             velocities, kinetic energy, pressure averages, the box
+// Bound by the latency of their loads, FP64 chains and grid-wide sums: with a
+// launch per pass, one thread per group and the last block reading the
+// partial sums one block after another, 40 steps of 24,000 atoms took 12.9
+// ms; now 11.35 (refresh of the sorted coordinates folded into the launch
+// that moves the list's shifts included).
 constexpr double kAtmosp = 1.4584007e-05;           // atm in AKMA pressure units
 constexpr double kPatmos = 1.0 / kAtmosp;
 constexpr double kSurfaceTensionFactor = 98.6923;   // dyne/cm to atm A
@@ -743,6 +878,9 @@ struct PistonScalars {
   double cf_on[3], cf_half[3];
   double box_old[3];             // the box before the last step (for the list's shifts)
   double vfac, lp_vfac;          // patm / V and V pbfact atmosp of the step's box
+  // the last predictor-corrector pass, per component: displacement
+  // fa delta + fb delta_prev, position r + xr r + xd delta + xp delta_prev
+  double fa[3], fb[3], xr[3], xd[3], xp[3];
   unsigned long long rngpos;     // normals drawn per piston degree of freedom
   unsigned counter, pad;
 };
@@ -763,33 +901,6 @@ struct PistonArgs {
   double ke_ref;
   int crystal, dof, use_nh, use_old, const_st, hol;
 };
-
-template <int N>
-__device__ void block_partials_n(const double (&v)[N], double *partials) {
-  __shared__ double sh[N][kThreads / 32];
-#pragma unroll
-  for (int k = 0; k < N; ++k) {
-    const double s = warp_sum(v[k]);
-    if ((threadIdx.x & 31) == 0) sh[k][threadIdx.x >> 5] = s;
-  }
-  __syncthreads();
-  if (threadIdx.x < N) {
-    double s = 0;
-    for (int w = 0; w < kThreads / 32; ++w) s += sh[threadIdx.x][w];
-    partials[N * blockIdx.x + threadIdx.x] = s;
-  }
-}
-
-// totals of the N partials of every block, in block order, into tot[]
-template <int N>
-__device__ void sum_partials_n(const double *partials, double *tot) {
-  if (threadIdx.x < N) {
-    double s = 0;
-    for (int b = 0; b < (int)gridDim.x; ++b) s += partials[N * b + threadIdx.x];
-    tot[threadIdx.x] = s;
-  }
-  __syncthreads();
-}
 
 // piston move of one predictor-corrector pass (one thread)
 // (UpdateLangevinPistonKernel, src/CudaLangevinPistonIntegrator.cu:1297-1452)
@@ -871,238 +982,255 @@ __device__ void lp_pass_start(const Common &c, const PistonArgs &a, double ke0, 
   piston_update(c.sc, a.use_old ? ke1 : ke0, a.ke_ref, dt);
 }
 
-__global__ void __launch_bounds__(kThreads) lp_half_kernel(Common c, PistonArgs a) {
-  if (*c.err) return;
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+// One pass of the predictor-corrector for all atoms at once: with c the
+// (thermostat + box) damping of a component,
+//   v = (delta_prev + d) / (2 dt),  d <- delta - c v,  x <- r + d + h (r + x) / 2
+// keeps d = A delta + B delta_prev and x = r + R r + D delta + P delta_prev
+// with the same factors for every atom.  Advances the factors and forms what
+// the pass sums over the atoms from the sums over m delta delta,
+// m delta delta_prev and m delta_prev delta_prev: the pressure's kinetic term
+// of d, and the on-step kinetic energy of v.
+struct PassSums {
+  const double *dd, *pp;  // xx xy xz yy yz zz of sum m d d / dt^2, sum m p p / dt^2
+  const double *dp;       // 3x3 of sum m d p / dt^2
+};
+__device__ __forceinline__ int sym(int u, int w) {  // index of (u, w) in xx xy xz yy yz zz
+  return u <= w ? (u == 0 ? w : u + w + 1) : (w == 0 ? u : u + w + 1);
+}
+__device__ void lp_pass(const PistonArgs &a, const Scalars *sc, const PassSums &S, double dt,
+                        double (&kin)[9], double &kon) {
+  PistonScalars *ps = a.ps;
+  const double nh = a.use_nh ? dt * dt * sc->piston_v : 0.0, fact = 0.5 / dt;
+  kon = 0.0;
+  for (int u = 0; u < 3; ++u) {
+    const double A = ps->fa[u], B = 1.0 + ps->fb[u], h = 0.5 * ps->cf_half[u];
+    kon += B * B * S.pp[sym(u, u)] + 2.0 * A * B * S.dp[4 * u] + A * A * S.dd[sym(u, u)];
+    const double f = (nh + dt * ps->cf_on[u]) * fact;
+    ps->fa[u] = 1.0 - f * A;
+    ps->fb[u] = -f * B;
+    ps->xr[u] = h * (2.0 + ps->xr[u]);
+    ps->xd[u] = ps->fa[u] + h * ps->xd[u];
+    ps->xp[u] = ps->fb[u] + h * ps->xp[u];
+  }
+  kon *= 0.5 * fact * fact * dt * dt;
+  for (int u = 0; u < 3; ++u)
+    for (int w = 0; w < 3; ++w)
+      kin[3 * u + w] = ps->fa[u] * ps->fa[w] * S.dd[sym(u, w)] +
+                       ps->fa[u] * ps->fb[w] * S.dp[3 * u + w] +
+                       ps->fb[u] * ps->fa[w] * S.dp[3 * w + u] +
+                       ps->fb[u] * ps->fb[w] * S.pp[sym(u, w)];
+}
+
+template <int W>
+__global__ void __launch_bounds__(kThreads) lp_half_kernel(Common c, PistonArgs a, int passes) {
+  constexpr int K = 4 / W;
+  const unsigned err = *c.err;
   const double dt = c.dt, dt2 = dt * dt, idt = 1.0 / dt;
-  // [0..8] constraint virial, [9..17] sum d d m/dt^2 of the new half step,
-  // [18..26] the same of the previous half step, [27..28] the kinetic
-  // energy of the first predictor-corrector pass
-  double v[29];
+  const GroupLane<W> G(c);
+  double4 x[K], vm[K], dp[K];
+  int slot[K];
 #pragma unroll
-  for (int k = 0; k < 29; ++k) v[k] = 0.0;
-  if (g < c.ngroups) {
-    int at[4];
-    const int m = group_atoms(c, g, at);
-    const int2 meta = c.gmeta[g];
-    double4 x[4], vm[4], dp[4];
-    int slot[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (k < m) {
-        const int i = at[k];
-        x[k] = c.coords[i];
-        vm[k] = c.vel[i];
-        dp[k] = c.dprev[i];
-        slot[k] = c.glo2loc[i];
-      }
+  for (int j = 0; j < K; ++j) {
+    x[j] = vm[j] = dp[j] = make_double4(0.0, 0.0, 0.0, 0.0);
+    slot[j] = 0;
+    if (G.on[j]) {
+      const int i = G.at[j];
+      x[j] = c.coords[i];
+      vm[j] = c.vel[i];
+      dp[j] = c.dprev[i];
+      slot[j] = c.glo2loc[i];
     }
-    d3 o[4], n[4], n0[4], du[4];
+  }
+  long long gi[K][3];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (k < m) {
-        const d3 gr = mk((double)c.force[slot[k]] * kInvForceScale,
-                         (double)c.force[c.stride + slot[k]] * kInvForceScale,
-                         (double)c.force[2 * c.stride + slot[k]] * kInvForceScale);
-        o[k] = xyz(x[k]);
-        du[k] = xyz(dp[k]) - (dt2 * vm[k].w) * gr;
-        n[k] = o[k] + du[k];
-        n0[k] = n[k];
-      }
+  for (int j = 0; j < K; ++j) {
+    if (G.on[j]) {
+      gi[j][0] = c.force[slot[j]];
+      gi[j][1] = c.force[c.stride + slot[j]];
+      gi[j][2] = c.force[2 * c.stride + slot[j]];
     }
-    if (a.hol) apply_constraint(meta.x, m, o, n, c.sk, c.shake_p, meta.y);
+  }
+  if (err) return;
+  d3 o[K], n[K], n0[K], du[K];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (k < m) {
-        const int i = at[k];
-        const double f = 1.0 / (dt2 * vm[k].w);
-        d3 d = du[k];
-        if (a.hol) {
-          // constraint force m (x_constrained - x_free) / dt^2 and its virial
-          // (ComputeHolonomicConstraintForces/VirialKernel)
-          const d3 fc = mk(f * (n[k].x - o[k].x - du[k].x), f * (n[k].y - o[k].y - du[k].y),
-                           f * (n[k].z - o[k].z - du[k].z));
-          const double r[3] = {o[k].x, o[k].y, o[k].z}, q[3] = {fc.x, fc.y, fc.z};
+  for (int j = 0; j < K; ++j) {
+    o[j] = xyz(x[j]);
+    du[j] = mk(0.0, 0.0, 0.0);
+    if (G.on[j]) {  // the slots are cleared for the next force evaluation
+      c.force[slot[j]] = 0;
+      c.force[c.stride + slot[j]] = 0;
+      c.force[2 * c.stride + slot[j]] = 0;
+      const d3 gr = mk((double)gi[j][0] * kInvForceScale, (double)gi[j][1] * kInvForceScale,
+                       (double)gi[j][2] * kInvForceScale);
+      du[j] = xyz(dp[j]) - (dt2 * vm[j].w) * gr;
+    }
+    n[j] = o[j] + du[j];
+    n0[j] = n[j];
+  }
+  if (a.hol) G.constrain(c, o, n);
+  // [0..8] constraint virial; sums over m / dt^2: [9..14] d d, [15..20]
+  // delta_prev delta_prev, [21..29] d delta_prev; [30] twice the on-step
+  // kinetic energy
+  double v[31];
 #pragma unroll
-          for (int u = 0; u < 3; ++u)
+  for (int k = 0; k < 31; ++k) v[k] = 0.0;
 #pragma unroll
-            for (int w = 0; w < 3; ++w) v[3 * u + w] += r[u] * q[w];
-          d = n[k] - o[k];
-        }
-        const double dd[3] = {d.x, d.y, d.z}, pp[3] = {dp[k].x, dp[k].y, dp[k].z};
+  for (int j = 0; j < K; ++j) {
+    if (G.on[j]) {
+      const double f = 1.0 / (dt2 * vm[j].w);
+      d3 d = du[j];
+      if (a.hol) {
+        // constraint force m (x_constrained - x_free) / dt^2 and its virial
+        // (ComputeHolonomicConstraintForces/VirialKernel)
+        const d3 fc = mk(f * (n[j].x - o[j].x - du[j].x), f * (n[j].y - o[j].y - du[j].y),
+                         f * (n[j].z - o[j].z - du[j].z));
+        const double r[3] = {o[j].x, o[j].y, o[j].z}, q[3] = {fc.x, fc.y, fc.z};
 #pragma unroll
         for (int u = 0; u < 3; ++u)
 #pragma unroll
-          for (int w = 0; w < 3; ++w) {
-            v[9 + 3 * u + w] += f * dd[u] * dd[w];
-            v[18 + 3 * u + w] += f * pp[u] * pp[w];
-          }
-        c.ref[i] = x[k];
-        c.delta[i] = make_double4(d.x, d.y, d.z, 0.0);
-        c.dpred[i] = make_double4(d.x, d.y, d.z, 0.0);
-        const d3 xn = o[k] + d;
-        c.coords[i] = make_double4(a.hol ? n[k].x : xn.x, a.hol ? n[k].y : xn.y,
-                                   a.hol ? n[k].z : xn.z, x[k].w);
-        // a constraint pass adds its displacement over dt to the velocities
-        // (src/CudaHolonomicConstraint.cu:94-106): the first pass's on-step
-        // kinetic energy sees it
-        const d3 vn = xyz(vm[k]) + idt * (n[k] - n0[k]);
-        c.vel[i] = make_double4(vn.x, vn.y, vn.z, vm[k].w);
-        const d3 u1 = idt * xyz(dp[k]), u2 = idt * d;
-        const double kon = 0.5 * dot(vn, vn) / vm[k].w;
-        v[27] += (0.5 * dot(u1, u1) / vm[k].w + kon + 0.5 * dot(u2, u2) / vm[k].w) / 3.0;
-        v[28] += kon;
+          for (int w = 0; w < 3; ++w) v[3 * u + w] += r[u] * q[w];
+        d = n[j] - o[j];
       }
+      const double dd[3] = {d.x, d.y, d.z}, pp[3] = {dp[j].x, dp[j].y, dp[j].z};
+      int k = 0;
+#pragma unroll
+      for (int u = 0; u < 3; ++u)
+#pragma unroll
+        for (int w = u; w < 3; ++w, ++k) {
+          v[9 + k] += f * dd[u] * dd[w];
+          v[15 + k] += f * pp[u] * pp[w];
+        }
+#pragma unroll
+      for (int u = 0; u < 3; ++u)
+#pragma unroll
+        for (int w = 0; w < 3; ++w) v[21 + 3 * u + w] += f * dd[u] * pp[w];
+      c.delta[G.at[j]] = make_double4(d.x, d.y, d.z, 0.0);
+      // a constraint pass adds its displacement over dt to the velocities
+      // (src/CudaHolonomicConstraint.cu:94-106): the first pass's on-step
+      // kinetic energy sees it
+      const d3 vn = xyz(vm[j]) + idt * (n[j] - n0[j]);
+      v[30] += dot(vn, vn) / vm[j].w;
     }
   }
-  block_partials_n<29>(v, a.partials);
+  block_partials_n<31>(v, a.partials);
   if (is_last_block(&a.ps->counter)) {
-    __shared__ double tot[29];
-    sum_partials_n<29>(a.partials, tot);
+    __shared__ double tot[31];
+    sum_partials_n<31>(a.partials, tot);
     if (threadIdx.x == 0) {
       PistonScalars *ps = a.ps;
+      const PassSums sums{tot + 9, tot + 15, tot + 21};
       const double V = ps->box[0] * ps->box[1] * ps->box[2];
       ps->vfac = kPatmos / V;
       ps->lp_vfac = V * a.pbfact * kAtmosp;
-      for (int k = 0; k < 9; ++k) {
-        ps->vir[k] = (double)a.vir_fixed[k] * kInvEnergyScale + tot[k];
-        const double kin = 0.5 * (tot[9 + k] + tot[18 + k]);
-        ps->p[k] = ps->vfac * (kin + ps->vir[k]);
-        ps->dp[k] = ps->p[k] - ps->pref[k];
-      }
+      for (int u = 0; u < 3; ++u)
+        for (int w = 0; w < 3; ++w) {
+          const int k = 3 * u + w, q = sym(u, w);
+          ps->vir[k] = (double)a.vir_fixed[k] * kInvEnergyScale + tot[k];
+          const double kin = 0.5 * (sums.dd[q] + sums.pp[q]);
+          ps->p[k] = ps->vfac * (kin + ps->vir[k]);
+          ps->dp[k] = ps->p[k] - ps->pref[k];
+        }
       ps->pscalar = (ps->p[0] + ps->p[4] + ps->p[8]) / 3.0;
       if (a.const_st) {
         ps->pref[0] = ps->pref[8] - a.st / ps->box[2];
         ps->pref[4] = ps->pref[0];
       }
-      for (int k = 0; k < 9; ++k) ps->dp_static[k] = ps->dp[k] - 0.25 * ps->vfac * tot[9 + k];
+      for (int u = 0; u < 3; ++u)
+        for (int w = 0; w < 3; ++w)
+          ps->dp_static[3 * u + w] = ps->dp[3 * u + w] - 0.25 * ps->vfac * sums.dd[sym(u, w)];
       c.sc->piston_v_prev = c.sc->piston_v;
       c.sc->piston_f_prev = c.sc->piston_f;
-      lp_pass_start(c, a, tot[27], tot[28], dt);
+      for (int u = 0; u < 3; ++u) {
+        ps->fa[u] = ps->xd[u] = 1.0;
+        ps->fb[u] = ps->xr[u] = ps->xp[u] = 0.0;
+      }
+      // half-step kinetic energies of both sides (1/2 m u^2 with u over dt)
+      const double kp = 0.5 * (sums.pp[0] + sums.pp[3] + sums.pp[5]);
+      double kd = 0.5 * (sums.dd[0] + sums.dd[3] + sums.dd[5]);
+      double kon = 0.5 * tot[30], kin[9];
+      for (int pass = 0; pass < passes; ++pass) {
+        lp_pass_start(c, a, (kp + kon + kd) / 3.0, kon, dt);
+        lp_pass(a, c.sc, sums, dt, kin, kon);
+        for (int k = 0; k < 9; ++k) ps->dp[k] = ps->dp_static[k] + 0.25 * ps->vfac * kin[k];
+        kd = 0.5 * (kin[0] + kin[4] + kin[8]);
+      }
       ps->counter = 0;
     }
   }
 }
 
-// predictor-corrector pass over atoms: atoms follow piston and thermostat;
-// the last block forms the new pressure difference and, when another pass
-// follows (`more`), starts it from the kinetic energy of the new velocities
-__global__ void __launch_bounds__(kThreads) lp_pc_kernel(Common c, PistonArgs a, int natom,
-                                                         int more) {
-  if (*c.err) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const double dt = c.dt, dt2 = dt * dt, idt = 1.0 / dt, fact = 0.5 / dt;
-  const PistonScalars *ps = a.ps;
-  const double nh = a.use_nh ? dt2 * c.sc->piston_v : 0.0;
-  // [0..8] sum d d m/dt^2 of the predicted half step, [9..10] kinetic energy
-  double v[11];
-#pragma unroll
-  for (int k = 0; k < 11; ++k) v[k] = 0.0;
-  if (i < natom) {
-    const d3 dprev = xyz(c.dprev[i]), dpred = xyz(c.dpred[i]), d = xyz(c.delta[i]);
-    const d3 r = xyz(c.ref[i]);
-    const double4 x = c.coords[i];
-    const d3 u = fact * (dprev + dpred);
-    const d3 np = mk(d.x - (nh + dt * ps->cf_on[0]) * u.x, d.y - (nh + dt * ps->cf_on[1]) * u.y,
-                     d.z - (nh + dt * ps->cf_on[2]) * u.z);
-    c.dpred[i] = make_double4(np.x, np.y, np.z, 0.0);
-    const double im = c.vel[i].w;
-    c.vel[i] = make_double4(u.x, u.y, u.z, im);
-    const d3 h = 0.5 * (r + xyz(x));
-    c.coords[i] = make_double4(r.x + np.x + ps->cf_half[0] * h.x, r.y + np.y + ps->cf_half[1] * h.y,
-                               r.z + np.z + ps->cf_half[2] * h.z, x.w);
-    const double f = 1.0 / (dt2 * im);
-    const double nn[3] = {np.x, np.y, np.z};
-#pragma unroll
-    for (int p = 0; p < 3; ++p)
-#pragma unroll
-      for (int q = 0; q < 3; ++q) v[3 * p + q] = f * nn[p] * nn[q];
-    if (more) {
-      const d3 u1 = idt * dprev, u2 = idt * np;
-      const double kon = 0.5 * dot(u, u) / im;
-      v[9] = (0.5 * dot(u1, u1) / im + kon + 0.5 * dot(u2, u2) / im) / 3.0;
-      v[10] = kon;
-    }
-  }
-  block_partials_n<11>(v, a.partials);
-  if (is_last_block(&a.ps->counter)) {
-    __shared__ double tot[11];
-    sum_partials_n<11>(a.partials, tot);
-    if (threadIdx.x == 0) {
-      for (int k = 0; k < 9; ++k) a.ps->dp[k] = a.ps->dp_static[k] + 0.25 * a.ps->vfac * tot[k];
-      if (more) lp_pass_start(c, a, tot[9], tot[10], dt);
-      a.ps->counter = 0;
-    }
-  }
-}
-
+template <int W>
 __global__ void __launch_bounds__(kThreads) lp_final_kernel(Common c, PistonArgs a) {
-  if (*c.err) return;
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr int K = 4 / W;
+  const unsigned err = *c.err;
   const double dt = c.dt, dt2 = dt * dt, idt = 1.0 / dt, fact = 0.5 / dt;
+  const PistonScalars *cs = a.ps;
+  const GroupLane<W> G(c);
+  d3 o[K], n[K], dp[K], dn[K];
+  double q[K], im[K];
+#pragma unroll
+  for (int j = 0; j < K; ++j) {
+    o[j] = n[j] = dp[j] = dn[j] = mk(0.0, 0.0, 0.0);
+    q[j] = im[j] = 0.0;
+    if (G.on[j]) {
+      const int i = G.at[j];
+      const double4 x = c.coords[i];
+      o[j] = xyz(x);
+      q[j] = x.w;
+      dp[j] = xyz(c.dprev[i]);
+      dn[j] = xyz(c.delta[i]);
+      im[j] = c.vel[i].w;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < K; ++j) {  // the positions and displacements of the last pass
+    const d3 d = dn[j], p = dp[j];
+    n[j] = o[j] + mk(cs->xr[0] * o[j].x + cs->xd[0] * d.x + cs->xp[0] * p.x,
+                     cs->xr[1] * o[j].y + cs->xd[1] * d.y + cs->xp[1] * p.y,
+                     cs->xr[2] * o[j].z + cs->xd[2] * d.z + cs->xp[2] * p.z);
+    dn[j] = mk(cs->fa[0] * d.x + cs->fb[0] * p.x, cs->fa[1] * d.y + cs->fb[1] * p.y,
+               cs->fa[2] * d.z + cs->fb[2] * p.z);
+  }
+  if (err) return;
+  if (a.hol) {
+    // the new positions onto the constraints, the reference positions
+    // scaled with the box and constrained against the new ones, the
+    // displacement between them (src/CudaLangevinPistonIntegrator.cu:1955-1980)
+    G.constrain(c, o, n);
+    d3 rs[K];
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const d3 h = 0.5 * (o[j] + n[j]);
+      rs[j] = o[j] + mk(cs->cf_half[0] * h.x, cs->cf_half[1] * h.y, cs->cf_half[2] * h.z);
+    }
+    G.constrain(c, n, rs);
+#pragma unroll
+    for (int j = 0; j < K; ++j) dn[j] = n[j] - rs[j];
+  }
   // [0] 3-term kinetic energy, [1] on-step, [2..10] sum (d d + dp dp) m/dt^2
   double v[11];
 #pragma unroll
   for (int k = 0; k < 11; ++k) v[k] = 0.0;
-  if (g < c.ngroups) {
-    int at[4];
-    const int m = group_atoms(c, g, at);
-    const int2 meta = c.gmeta[g];
-    d3 o[4], n[4], dp[4], dn[4], rs[4];
-    double q[4], im[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (k < m) {
-        const int i = at[k];
-        o[k] = xyz(c.ref[i]);
-        const double4 x = c.coords[i];
-        n[k] = xyz(x);
-        q[k] = x.w;
-        dp[k] = xyz(c.dprev[i]);
-        dn[k] = xyz(c.dpred[i]);
-        im[k] = c.vel[i].w;
-      }
-    }
-    if (a.hol) {
-      // the new positions onto the constraints, the reference positions
-      // scaled with the box and constrained against the new ones, the
-      // displacement between them (src/CudaLangevinPistonIntegrator.cu:1955-1980)
-      apply_constraint(meta.x, m, o, n, c.sk, c.shake_p, meta.y);
-      const PistonScalars *ps = a.ps;
+  for (int j = 0; j < K; ++j) {
+    if (G.on[j]) {
+      const int i = G.at[j];
+      const d3 d = dn[j];
+      const d3 u = fact * (d + dp[j]);
+      const d3 u1 = idt * dp[j], u2 = idt * d;
+      const double kon = 0.5 * dot(u, u) / im[j];
+      v[0] += (0.5 * dot(u1, u1) / im[j] + kon + 0.5 * dot(u2, u2) / im[j]) / 3.0;
+      v[1] += kon;
+      const double f = 1.0 / (dt2 * im[j]);
+      const double dd[3] = {d.x, d.y, d.z}, pp[3] = {dp[j].x, dp[j].y, dp[j].z};
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if (k < m) {
-          const d3 h = 0.5 * (o[k] + n[k]);
-          rs[k] = o[k] + mk(ps->cf_half[0] * h.x, ps->cf_half[1] * h.y, ps->cf_half[2] * h.z);
-        }
-      }
-      apply_constraint(meta.x, m, n, rs, c.sk, c.shake_p, meta.y);
+      for (int s = 0; s < 3; ++s)
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if (k < m) dn[k] = n[k] - rs[k];
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (k < m) {
-        const int i = at[k];
-        const d3 d = dn[k];
-        const d3 u = fact * (d + dp[k]);
-        const d3 u1 = idt * dp[k], u2 = idt * d;
-        const double kon = 0.5 * dot(u, u) / im[k];
-        v[0] += (0.5 * dot(u1, u1) / im[k] + kon + 0.5 * dot(u2, u2) / im[k]) / 3.0;
-        v[1] += kon;
-        const double f = 1.0 / (dt2 * im[k]);
-        const double dd[3] = {d.x, d.y, d.z}, pp[3] = {dp[k].x, dp[k].y, dp[k].z};
-#pragma unroll
-        for (int s = 0; s < 3; ++s)
-#pragma unroll
-          for (int w = 0; w < 3; ++w) v[2 + 3 * s + w] += f * (dd[s] * dd[w] + pp[s] * pp[w]);
-        c.delta[i] = make_double4(d.x, d.y, d.z, 0.0);
-        c.dprev[i] = make_double4(d.x, d.y, d.z, 0.0);
-        c.vel[i] = make_double4(u.x, u.y, u.z, im[k]);
-        c.coords[i] = make_double4(n[k].x, n[k].y, n[k].z, q[k]);
-        c.xyzq[i] = make_float4((float)n[k].x, (float)n[k].y, (float)n[k].z, (float)q[k]);
-      }
+        for (int w = 0; w < 3; ++w) v[2 + 3 * s + w] += f * (dd[s] * dd[w] + pp[s] * pp[w]);
+      c.dprev[i] = make_double4(d.x, d.y, d.z, 0.0);
+      c.vel[i] = make_double4(u.x, u.y, u.z, im[j]);
+      c.coords[i] = make_double4(n[j].x, n[j].y, n[j].z, q[j]);
+      c.xyzq[i] = make_float4((float)n[j].x, (float)n[j].y, (float)n[j].z, (float)q[j]);
     }
   }
   block_partials_n<11>(v, a.partials);
@@ -1179,7 +1307,7 @@ struct IntegratorState {
   DeviceArray<int4> groups;
   DeviceArray<int2> gmeta;
   DeviceArray<float4> shake_p;
-  DeviceArray<double4> dprev, delta, dpred, ref;
+  DeviceArray<double4> dprev, delta;
   DeviceArray<Scalars> sc;
   DeviceArray<double> partials;
   int ngroups = 0, natom = 0;
@@ -1303,8 +1431,6 @@ void CudaIntegrator::buildGroups() {
   upload(S.shake_p, t.shake_p);
   S.dprev.alloc(n);
   S.delta.alloc(n);
-  S.dpred.alloc(n);
-  S.ref.alloc(n);
   APO_CUDA(cudaMemset(S.dprev.p, 0, n * sizeof(double4)));
   APO_CUDA(cudaMemset(S.delta.p, 0, n * sizeof(double4)));
   S.sc.alloc(1);
@@ -1339,8 +1465,6 @@ void CudaIntegrator::buildGroups() {
   c.vel = m_Ctx->velMass();
   c.dprev = S.dprev.p;
   c.delta = S.delta.p;
-  c.dpred = S.dpred.p;
-  c.ref = S.ref.p;
   c.xyzq = m_Ctx->xyzq();
   c.force = fm->forceFixed();
   c.stride = fm->forceStride();
@@ -1721,7 +1845,7 @@ void CudaLangevinThermostatIntegrator::stepKernels(cudaStream_t s) {
 // ------------------------------------------------------------- Nose-Hoover
 
 CudaNoseHooverIntegrator::CudaNoseHooverIntegrator(double ps) : CudaIntegrator(ps) {
-  m_KernelsPerStep = 5;
+  m_KernelsPerStep = 2;
 }
 
 void CudaNoseHooverIntegrator::setNoseHooverPistonMass(double m) {
@@ -1762,11 +1886,13 @@ void CudaNoseHooverIntegrator::stepKernels(cudaStream_t s) {
   IntegratorState &S = *m_S;
   const double ke_ref = 0.5 * m_Ctx->getDegreesOfFreedom() * kBoltz * m_RefT;
   const int old = m_OldT ? 1 : 0;
-  nh_half_kernel<<<S.blocks_groups, kThreads, 0, s>>>(S.c, ke_ref, old);
-  nh_pc_kernel<true><<<S.blocks_atoms, kThreads, 0, s>>>(S.c, S.natom, ke_ref, old);
-  nh_pc_kernel<true><<<S.blocks_atoms, kThreads, 0, s>>>(S.c, S.natom, ke_ref, old);
-  nh_pc_kernel<false><<<S.blocks_atoms, kThreads, 0, s>>>(S.c, S.natom, ke_ref, old);
-  nh_final_kernel<<<S.blocks_groups, kThreads, 0, s>>>(S.c, ke_ref, old);
+  if (S.ngroups <= kFourLaneGroups) {
+    nh_half_kernel<4><<<S.blocks_lanes, kThreads, 0, s>>>(S.c, ke_ref, old);
+    nh_final_kernel<4><<<S.blocks_lanes, kThreads, 0, s>>>(S.c, ke_ref, old);
+  } else {
+    nh_half_kernel<1><<<S.blocks_groups, kThreads, 0, s>>>(S.c, ke_ref, old);
+    nh_final_kernel<1><<<S.blocks_groups, kThreads, 0, s>>>(S.c, ke_ref, old);
+  }
   APO_LAUNCH_CHECK();
 }
 
@@ -1781,7 +1907,7 @@ struct PistonState {
 CudaLangevinPistonIntegrator::CudaLangevinPistonIntegrator(double ps) : CudaIntegrator(ps) {
   std::random_device rd;
   m_Seed = rd();
-  m_KernelsPerStep = 3 + m_MaxPC;
+  m_KernelsPerStep = 3;
 }
 
 CudaLangevinPistonIntegrator::~CudaLangevinPistonIntegrator() = default;
@@ -1868,7 +1994,7 @@ void CudaLangevinPistonIntegrator::setMaxPredictorCorrectorIterations(int n) {
   if (n < 1)
     throw std::invalid_argument("setMaxPredictorCorrectorIterations: at least one pass is needed");
   m_MaxPC = n;
-  m_KernelsPerStep = 3 + m_MaxPC;
+  m_KernelsPerStep = 3;
   clearGraphs();
 }
 
@@ -1972,7 +2098,7 @@ void CudaLangevinPistonIntegrator::initialize() {
   PistonState &P = *m_P;
   P.ps.alloc(1);
   P.rng.alloc(3);
-  P.partials.alloc((size_t)32 * std::max(S.blocks_groups, S.blocks_atoms) + 32);
+  P.partials.alloc((size_t)32 * std::max(S.blocks_groups, S.blocks_lanes) + 32);
   PistonScalars h{};
   const auto &box = fm->getBoxDimensions();
   for (int d = 0; d < 3; ++d) h.box[d] = h.box_pred[d] = box[d];
@@ -2057,10 +2183,13 @@ void CudaLangevinPistonIntegrator::stepKernels(cudaStream_t s) {
   a.use_old = m_OldT ? 1 : 0;
   a.const_st = m_ConstST ? 1 : 0;
   a.hol = m_Ctx->isUsingHolonomicConstraints() ? 1 : 0;
-  lp_half_kernel<<<S.blocks_groups, kThreads, 0, s>>>(S.c, a);
-  for (int k = 0; k < m_MaxPC; ++k)
-    lp_pc_kernel<<<S.blocks_atoms, kThreads, 0, s>>>(S.c, a, S.natom, k + 1 < m_MaxPC ? 1 : 0);
-  lp_final_kernel<<<S.blocks_groups, kThreads, 0, s>>>(S.c, a);
+  if (S.ngroups <= kFourLaneGroups) {
+    lp_half_kernel<4><<<S.blocks_lanes, kThreads, 0, s>>>(S.c, a, m_MaxPC);
+    lp_final_kernel<4><<<S.blocks_lanes, kThreads, 0, s>>>(S.c, a);
+  } else {
+    lp_half_kernel<1><<<S.blocks_groups, kThreads, 0, s>>>(S.c, a, m_MaxPC);
+    lp_final_kernel<1><<<S.blocks_groups, kThreads, 0, s>>>(S.c, a);
+  }
   APO_LAUNCH_CHECK();
   const char *ps = reinterpret_cast<const char *>(P.ps.p);
   fm->neighborList().rescale_box_device(
@@ -2069,9 +2198,9 @@ void CudaLangevinPistonIntegrator::stepKernels(cudaStream_t s) {
 }
 
 void CudaLangevinPistonIntegrator::forcesForStep(cudaStream_t s) {
-  // forces and virial; the sorted coordinates refreshed from the FP64 state
-  // the step kernels wrote, the gradient slots cleared
-  m_Ctx->getForceManager()->calcForce(m_Ctx->xyzq(), false, true, s, /*clear=*/true);
+  // forces and virial; the step kernels have cleared the gradient slots and
+  // refreshed the sorted coordinates (the list build does at a segment's start)
+  m_Ctx->getForceManager()->calcForce(m_Ctx->xyzq(), false, true, s, /*clear=*/false);
 }
 
 void CudaLangevinPistonIntegrator::adoptBox() {

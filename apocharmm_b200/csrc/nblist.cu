@@ -251,21 +251,30 @@ __global__ void origin_kernel(const float4 *__restrict__ xyzq, const int *__rest
 }
 
 // a new box for the built list: slot_off = k L - origin becomes k L' - origin
-// (k recovered from the old box; the origins stay)
+// (k recovered from the old box; the origins stay), and the sorted
+// coordinates of the new positions in the new box
 __global__ void rescale_dev_kernel(double4 *__restrict__ slot_off,
                                    const float4 *__restrict__ cl_origin,
                                    const double *__restrict__ L0, const double *__restrict__ L1,
-                                   const unsigned *__restrict__ err, const int *__restrict__ counts) {
+                                   const unsigned *__restrict__ err, const int *__restrict__ counts,
+                                   const double4 *__restrict__ coords,
+                                   const int *__restrict__ perm, float4 *__restrict__ xyzq_s) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (*err || s >= counts[0]) return;
+  const int g = perm[s];
   const float4 o = cl_origin[s / kTile];
   double4 v = slot_off[s];
+  double4 c = make_double4(0.0, 0.0, 0.0, 0.0);
+  if (g >= 0) c = coords[g];
   const double kx = rint((v.x + (double)o.x) / L0[0]), ky = rint((v.y + (double)o.y) / L0[1]),
                kz = rint((v.z + (double)o.z) / L0[2]);
   v.x = kx * L1[0] - (double)o.x;
   v.y = ky * L1[1] - (double)o.y;
   v.z = kz * L1[2] - (double)o.z;
   slot_off[s] = v;
+  xyzq_s[s] = g >= 0 ? make_float4((float)(c.x + v.x), (float)(c.y + v.y), (float)(c.z + v.z),
+                                   (float)c.w)
+                     : make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 // sorted, cluster-local coordinates (runs after every coordinate update)
@@ -743,8 +752,9 @@ void NeighborList::set_box(int sys, double Lx, double Ly, double Lz) {
 void NeighborList::rescale_box_device(const double *old_box, const double *new_box,
                                       const unsigned *err, cudaStream_t s) {
   if (m_sys_h.size() != 1) throw std::invalid_argument("NeighborList: one system only");
-  rescale_dev_kernel<<<(m_d.slot_cap + 255) / 256, 256, 0, s>>>(slot_off, cl_origin, old_box,
-                                                                new_box, err, counts);
+  if (!m_coords) throw std::runtime_error("NeighborList: no state coordinates attached");
+  rescale_dev_kernel<<<(m_d.slot_cap + 255) / 256, 256, 0, s>>>(
+      slot_off, cl_origin, old_box, new_box, err, counts, m_coords, perm, xyzq_s);
   APO_LAUNCH_CHECK();
 }
 

@@ -95,7 +95,8 @@ class NeighborList {
   void set_box(int sys, double Lx, double Ly, double Lz);
   // keep the built list under a new box: every slot's periodic shift k L
   // moves with the box (k kept), so the list stays valid between builds
-  // while the box changes a little every step; the old and new edges are
+  // while the box changes a little every step, and the sorted coordinates
+  // are refreshed in the new box; the old and new edges are
   // in device memory (3 doubles each; nothing happens once `err` is set)
   // and the device dims are left alone
   void rescale_box_device(const double *old_box, const double *new_box, const unsigned *err,
