@@ -18,14 +18,16 @@
 namespace apo {
 namespace {
 
-constexpr int kPlaneThreads = 512;
+constexpr int kPlaneThreadsMax = 1024;
 // dynamic shared memory a plane transform may use: the SM's 227 KB per
 // block less the kernels' static digit-reversal table
 constexpr size_t kPlaneSmemMax = 227 * 1024 - 1024;
 // the tensor-map argument of launches that move their slabs with plain loads
 const CUtensorMap kNoTensorMap{};
 constexpr int kPencilThreads = 256;
-constexpr int kPencilTX = 16;
+// a pencil slab's complex columns x planes: at most 24 x 256 (set_tiles), and
+// room to start it on 128 bytes
+constexpr size_t kPencilSmemMax = 24 * 256 * sizeof(float2) + 128;
 
 // ------------------------------------------------------------------------
 // B-spline weights (Essmann et al. recursion, the reference's calc_one_theta,
@@ -90,8 +92,11 @@ __device__ __forceinline__ double3 global_pos(const float4 &p, const float4 *ori
 // ------------------------------------------------------------------------
 // small DFTs
 // ------------------------------------------------------------------------
+// (every product and sum below is rounded where it is written, so that all
+// kernels that transform the same numbers get the same bits)
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+  return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)),
+                     __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x)));
 }
 
 // cos / sin of 2*pi*k/R for the radices used (exact mathematical constants)
@@ -118,127 +123,195 @@ __device__ __forceinline__ constexpr float rsin(int R, int k) {
        : 0.f;
 }
 
-// y_k = sum_q x_q exp(sign * 2 pi i q k / R)
-template <int R>
-__device__ __forceinline__ void dft(float2 (&x)[R], float sign) {
-  if (R == 2) {
-    float2 a = x[0], b = x[1];
-    x[0] = make_float2(a.x + b.x, a.y + b.y);
-    x[1] = make_float2(a.x - b.x, a.y - b.y);
-  } else if (R == 4) {
-    float2 s02 = make_float2(x[0].x + x[2].x, x[0].y + x[2].y);
-    float2 d02 = make_float2(x[0].x - x[2].x, x[0].y - x[2].y);
-    float2 s13 = make_float2(x[1].x + x[3].x, x[1].y + x[3].y);
-    float2 d13 = make_float2(x[1].x - x[3].x, x[1].y - x[3].y);
-    // sign * i * d13
-    float2 id13 = make_float2(-sign * d13.y, sign * d13.x);
-    x[0] = make_float2(s02.x + s13.x, s02.y + s13.y);
-    x[2] = make_float2(s02.x - s13.x, s02.y - s13.y);
-    x[1] = make_float2(d02.x + id13.x, d02.y + id13.y);
-    x[3] = make_float2(d02.x - id13.x, d02.y - id13.y);
-  } else {
-    float2 y[R];
+// y_k = sum_q x_q exp(+- 2 pi i q k / R), + when INV.  Each radix in its usual
+// factored form (real arithmetic shared between y_k and y_{R-k}; 6 as 2 x 3
+// and 8 as 2 x 4): 16 real additions for R = 4, 52 additions and 4
+// multiplications for R = 8, where the R^2 products of the definition are 256
+// multiply-adds.
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) {
+  return make_float2(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y));
+}
+__device__ __forceinline__ float2 csub(float2 a, float2 b) {
+  return make_float2(__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y));
+}
+// a + i b when INV, else a - i b
+template <bool INV>
+__device__ __forceinline__ float2 cadd_i(float2 a, float2 b) {
+  return INV ? make_float2(__fsub_rn(a.x, b.y), __fadd_rn(a.y, b.x))
+             : make_float2(__fadd_rn(a.x, b.y), __fsub_rn(a.y, b.x));
+}
+// b + s a, and b + i s a
+__device__ __forceinline__ float2 cfma(float s, float2 a, float2 b) {
+  return make_float2(__fmaf_rn(s, a.x, b.x), __fmaf_rn(s, a.y, b.y));
+}
+__device__ __forceinline__ float2 cfma_i(float s, float2 a, float2 b) {
+  return make_float2(__fmaf_rn(-s, a.y, b.x), __fmaf_rn(s, a.x, b.y));
+}
+
+template <bool INV>
+__device__ __forceinline__ void dft2(float2 &a, float2 &b) {
+  const float2 t = a;
+  a = cadd(t, b);
+  b = csub(t, b);
+}
+template <bool INV>
+__device__ __forceinline__ void dft3(float2 &x0, float2 &x1, float2 &x2) {
+  const float2 t = cadd(x1, x2), d = csub(x1, x2);
+  const float2 m = cfma(-0.5f, t, x0);
+  const float h = INV ? rsin(3, 1) : -rsin(3, 1);
+  x0 = cadd(x0, t);
+  x1 = cfma_i(h, d, m);
+  x2 = cfma_i(-h, d, m);
+}
+template <bool INV>
+__device__ __forceinline__ void dft4(float2 &x0, float2 &x1, float2 &x2, float2 &x3) {
+  const float2 s02 = cadd(x0, x2), d02 = csub(x0, x2), s13 = cadd(x1, x3), d13 = csub(x1, x3);
+  x0 = cadd(s02, s13);
+  x2 = csub(s02, s13);
+  x1 = cadd_i<INV>(d02, d13);
+  x3 = cadd_i<!INV>(d02, d13);
+}
+
+template <int R, bool INV>
+__device__ __forceinline__ void dft(float2 (&x)[R]) {
+  if constexpr (R == 2) {
+    dft2<INV>(x[0], x[1]);
+  } else if constexpr (R == 3) {
+    dft3<INV>(x[0], x[1], x[2]);
+  } else if constexpr (R == 4) {
+    dft4<INV>(x[0], x[1], x[2], x[3]);
+  } else if constexpr (R == 6) {
+    // index maps q = 3 q1 + 2 q2, k = 3 k1 + 4 k2 (mod 6): no twiddles between
+    float2 a0 = x[0], b0 = x[3], a1 = x[2], b1 = x[5], a2 = x[4], b2 = x[1];
+    dft2<INV>(a0, b0);
+    dft2<INV>(a1, b1);
+    dft2<INV>(a2, b2);
+    dft3<INV>(a0, a1, a2);
+    dft3<INV>(b0, b1, b2);
+    x[0] = a0;
+    x[4] = a1;
+    x[2] = a2;
+    x[3] = b0;
+    x[1] = b1;
+    x[5] = b2;
+  } else if constexpr (R == 8) {
+    dft4<INV>(x[0], x[2], x[4], x[6]);
+    dft4<INV>(x[1], x[3], x[5], x[7]);
+    // odd half times exp(+- 2 pi i k / 8)
+    const float c = rcos(8, 1);
+    const float2 o1 = cadd_i<INV>(x[3], x[3]), o3 = cadd_i<!INV>(x[7], x[7]);
+    const float2 e0 = x[0], e1 = x[2], e2 = x[4], e3 = x[6], o0 = x[1], o2 = x[5];
+    x[0] = cadd(e0, o0);
+    x[4] = csub(e0, o0);
+    x[1] = cfma(c, o1, e1);
+    x[5] = cfma(-c, o1, e1);
+    x[2] = cadd_i<INV>(e2, o2);
+    x[6] = cadd_i<!INV>(e2, o2);
+    x[3] = cfma(-c, o3, e3);
+    x[7] = cfma(c, o3, e3);
+  } else {  // 5 and 7: pairs q, R - q
+    constexpr int H = R / 2;
+    float2 t[H], d[H];
 #pragma unroll
-    for (int k = 0; k < R; ++k) {
-      float re = 0.f, im = 0.f;
-#pragma unroll
-      for (int q = 0; q < R; ++q) {
-        const int idx = (q * k) % R;
-        const float c = rcos(R, idx), s = sign * rsin(R, idx);
-        re += x[q].x * c - x[q].y * s;
-        im += x[q].x * s + x[q].y * c;
-      }
-      y[k] = make_float2(re, im);
+    for (int q = 1; q <= H; ++q) {
+      t[q - 1] = cadd(x[q], x[R - q]);
+      d[q - 1] = csub(x[q], x[R - q]);
     }
+    const float2 x0 = x[0];
+    float2 y0 = x0;
 #pragma unroll
-    for (int k = 0; k < R; ++k) x[k] = y[k];
+    for (int q = 0; q < H; ++q) y0 = cadd(y0, t[q]);
+    x[0] = y0;
+#pragma unroll
+    for (int k = 1; k <= H; ++k) {
+      float2 m = x0, n = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int q = 1; q <= H; ++q) {
+        m = cfma(rcos(R, (q * k) % R), t[q - 1], m);
+        n = cfma(rsin(R, (q * k) % R), d[q - 1], n);
+      }
+      x[k] = cadd_i<INV>(m, n);
+      x[R - k] = cadd_i<!INV>(m, n);
+    }
   }
 }
 
-__device__ __forceinline__ float2 twiddle(const float2 *tw, int idx, float sign) {
-  float2 w = tw[idx];
-  if (sign > 0.f) w.y = -w.y;
+template <bool INV>
+__device__ __forceinline__ float2 twiddle(const float2 *tw, int idx) {
+  float2 w = __ldg(tw + idx);
+  if (INV) w.y = -w.y;
   return w;
 }
 
-// One decimation-in-frequency stage (butterfly, then twiddle) on sub-blocks
-// of length m of every line.  Lines start at buf + line*lstride; element e of
-// a line is at e*estride.  The twiddle index j k n/m stays below n.
-template <int R>
-__device__ void dif_stage(float2 *buf, int nlines, int lstride, int estride, int n, int m,
-                          FastDiv fpl, FastDiv fmr, const float2 *tw, float sign) {
-  const int mr = m / R, per_line = n / R, total = nlines * per_line, nm = n / m;
+// One stage on sub-blocks of length m of every line: decimation in frequency
+// (butterfly, then twiddle) or in time (twiddle, then butterfly).  Lines start
+// at buf + line * lstride; element e of a line is at e * estride.  The twiddle
+// index j k n/m stays below n.  Consecutive threads take consecutive lines:
+// their shared-memory accesses are lstride apart, free of bank conflicts for
+// columns (lstride 1; with consecutive threads along a line the z pencils,
+// estride 16, hit one bank with half a warp: 14.5 us a launch at 64^3 and 242
+// us at 216^3 against 11.2 and 65) and two-way at worst for packed rows (an odd
+// number of 16-byte units apart), whatever the stage's radix.
+template <int R, bool DIF, bool INV>
+__device__ __forceinline__ void fft_stage(float2 *buf, int nlines, FastDiv by_lines, int lstride,
+                                          int estride, int n, int m, FastDiv fmr, const float2 *tw) {
+  const int mr = m / R, total = nlines * (n / R), nm = n / m;
   for (int b = threadIdx.x; b < total; b += blockDim.x) {
-    const int line = (int)fdiv((unsigned)b, fpl), rem = b - line * per_line;
+    const int rem = (int)fdiv((unsigned)b, by_lines), line = b - rem * nlines;
     const int blk = (int)fdiv((unsigned)rem, fmr), j = rem - blk * mr;
     float2 *p = buf + line * lstride + (blk * m + j) * estride;
+    const int step = mr * estride;
     float2 x[R];
 #pragma unroll
-    for (int q = 0; q < R; ++q) x[q] = p[q * mr * estride];
-    dft<R>(x, sign);
-    if (j > 0) {
+    for (int q = 0; q < R; ++q) x[q] = p[q * step];
+    if (!DIF && j > 0) {
 #pragma unroll
-      for (int k = 1; k < R; ++k) x[k] = cmul(x[k], twiddle(tw, j * k * nm, sign));
+      for (int k = 1; k < R; ++k) x[k] = cmul(x[k], twiddle<INV>(tw, j * k * nm));
+    }
+    dft<R, INV>(x);
+    if (DIF && j > 0) {
+#pragma unroll
+      for (int k = 1; k < R; ++k) x[k] = cmul(x[k], twiddle<INV>(tw, j * k * nm));
     }
 #pragma unroll
-    for (int k = 0; k < R; ++k) p[k * mr * estride] = x[k];
+    for (int k = 0; k < R; ++k) p[k * step] = x[k];
   }
 }
 
-// One decimation-in-time stage (twiddle, then butterfly).
-template <int R>
-__device__ void dit_stage(float2 *buf, int nlines, int lstride, int estride, int n, int m,
-                          FastDiv fpl, FastDiv fmr, const float2 *tw, float sign) {
-  const int mr = m / R, per_line = n / R, total = nlines * per_line, nm = n / m;
-  for (int b = threadIdx.x; b < total; b += blockDim.x) {
-    const int line = (int)fdiv((unsigned)b, fpl), rem = b - line * per_line;
-    const int blk = (int)fdiv((unsigned)rem, fmr), j = rem - blk * mr;
-    float2 *p = buf + line * lstride + (blk * m + j) * estride;
-    float2 x[R];
-#pragma unroll
-    for (int k = 0; k < R; ++k) x[k] = p[k * mr * estride];
-    if (j > 0) {
-#pragma unroll
-      for (int k = 1; k < R; ++k) x[k] = cmul(x[k], twiddle(tw, j * k * nm, sign));
-    }
-    dft<R>(x, sign);
-#pragma unroll
-    for (int q = 0; q < R; ++q) p[q * mr * estride] = x[q];
-  }
-}
-
-template <bool DIF>
-__device__ __forceinline__ void stage(int R, float2 *buf, int nl, int ls, int es, int n, int m,
-                                      FastDiv fpl, FastDiv fmr, const float2 *tw, float sign) {
+template <bool DIF, bool INV>
+__device__ __forceinline__ void stage(int R, float2 *buf, int nl, FastDiv by_nl, int ls, int es,
+                                      int n, int m, FastDiv fmr, const float2 *tw) {
   switch (R) {
-    case 2: DIF ? dif_stage<2>(buf, nl, ls, es, n, m, fpl, fmr, tw, sign) : dit_stage<2>(buf, nl, ls, es, n, m, fpl, fmr, tw, sign); break;
-    case 3: DIF ? dif_stage<3>(buf, nl, ls, es, n, m, fpl, fmr, tw, sign) : dit_stage<3>(buf, nl, ls, es, n, m, fpl, fmr, tw, sign); break;
-    case 4: DIF ? dif_stage<4>(buf, nl, ls, es, n, m, fpl, fmr, tw, sign) : dit_stage<4>(buf, nl, ls, es, n, m, fpl, fmr, tw, sign); break;
-    case 5: DIF ? dif_stage<5>(buf, nl, ls, es, n, m, fpl, fmr, tw, sign) : dit_stage<5>(buf, nl, ls, es, n, m, fpl, fmr, tw, sign); break;
-    case 6: DIF ? dif_stage<6>(buf, nl, ls, es, n, m, fpl, fmr, tw, sign) : dit_stage<6>(buf, nl, ls, es, n, m, fpl, fmr, tw, sign); break;
-    case 7: DIF ? dif_stage<7>(buf, nl, ls, es, n, m, fpl, fmr, tw, sign) : dit_stage<7>(buf, nl, ls, es, n, m, fpl, fmr, tw, sign); break;
-    case 8: DIF ? dif_stage<8>(buf, nl, ls, es, n, m, fpl, fmr, tw, sign) : dit_stage<8>(buf, nl, ls, es, n, m, fpl, fmr, tw, sign); break;
+    case 2: fft_stage<2, DIF, INV>(buf, nl, by_nl, ls, es, n, m, fmr, tw); break;
+    case 3: fft_stage<3, DIF, INV>(buf, nl, by_nl, ls, es, n, m, fmr, tw); break;
+    case 4: fft_stage<4, DIF, INV>(buf, nl, by_nl, ls, es, n, m, fmr, tw); break;
+    case 5: fft_stage<5, DIF, INV>(buf, nl, by_nl, ls, es, n, m, fmr, tw); break;
+    case 6: fft_stage<6, DIF, INV>(buf, nl, by_nl, ls, es, n, m, fmr, tw); break;
+    case 7: fft_stage<7, DIF, INV>(buf, nl, by_nl, ls, es, n, m, fmr, tw); break;
+    case 8: fft_stage<8, DIF, INV>(buf, nl, by_nl, ls, es, n, m, fmr, tw); break;
     default: break;
   }
 }
 
 // natural order in, digit-reversed out
-__device__ void fft_dif(float2 *buf, int nl, int ls, int es, const FftAxis &a, const float2 *tw,
-                        float sign) {
+template <bool INV>
+__device__ void fft_dif(float2 *buf, int nl, FastDiv by_nl, int ls, int es, const FftAxis &a,
+                        const float2 *tw) {
   int m = a.n;
   for (int s = 0; s < a.nrad; ++s) {
-    stage<true>(a.radix[s], buf, nl, ls, es, a.n, m, a.per_line[s], a.dif_mr[s], tw, sign);
+    stage<true, INV>(a.radix[s], buf, nl, by_nl, ls, es, a.n, m, a.dif_mr[s], tw);
     __syncthreads();
     m /= a.radix[s];
   }
 }
 // digit-reversed in, natural order out
-__device__ void fft_dit(float2 *buf, int nl, int ls, int es, const FftAxis &a, const float2 *tw,
-                        float sign) {
+template <bool INV>
+__device__ void fft_dit(float2 *buf, int nl, FastDiv by_nl, int ls, int es, const FftAxis &a,
+                        const float2 *tw) {
   int m = 1;
   for (int s = a.nrad - 1; s >= 0; --s) {
     m *= a.radix[s];
-    stage<false>(a.radix[s], buf, nl, ls, es, a.n, m, a.per_line[s], a.dit_mr[s], tw, sign);
+    stage<false, INV>(a.radix[s], buf, nl, by_nl, ls, es, a.n, m, a.dit_mr[s], tw);
     __syncthreads();
   }
 }
@@ -412,7 +485,7 @@ __global__ void __launch_bounds__(128) spread_kernel(const float4 *__restrict__ 
 // The grid dimensions are read through a pointer (to the kernel parameter or
 // to the system's entry of the multi-system table), never copied: the FFT
 // stages index their per-stage divisors at run time.
-__global__ void __launch_bounds__(kPlaneThreads) plane_fwd_kernel(const __grid_constant__ PmeDims d0, int *__restrict__ qgrid,
+__global__ void __launch_bounds__(kPlaneThreadsMax) plane_fwd_kernel(const __grid_constant__ PmeDims d0, int *__restrict__ qgrid,
                                                                   float2 *__restrict__ cgrid,
                                                                   const float2 *__restrict__ twx,
                                                                   const float2 *__restrict__ twy,
@@ -433,31 +506,45 @@ __global__ void __launch_bounds__(kPlaneThreads) plane_fwd_kernel(const __grid_c
   const PmeDims &d = *dp;
   __shared__ short s_rev[256];  // x -> position in the digit-reversed row
   const int nx = d.nx, ny = d.ny, nxc = d.nxc, nxcp = d.nxcp, rowp = nx + 2, h = nx / 2;
-  int *plane = qgrid + (size_t)z * nx * ny;
+  // four points a thread and load (nx and ny are even, so a plane is a
+  // multiple of 16 bytes; the four points may run into the next row), two
+  // loads in flight, the first ones while the table is made
+  int4 *plane = reinterpret_cast<int4 *>(qgrid + (size_t)z * nx * ny);
+  const int total4 = nx * ny / 4;
+  int4 v[2];
+  const auto fetch = [&](int base) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = base + u * blockDim.x;
+      if (i < total4) v[u] = plane[i];
+    }
+  };
+  fetch(threadIdx.x);
   fill_rev_table(s_rev, d.ax, false);
   __syncthreads();
-  // four loads in flight per thread before any store (latency-bound loop)
-  const int total = nx * ny;
-  for (int base = threadIdx.x; base < total; base += 4 * blockDim.x) {
-    int v[4];
+  for (int base = threadIdx.x; base < total4; base += 2 * blockDim.x) {
+    if (base != (int)threadIdx.x) fetch(base);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int idx = base + u * blockDim.x;
-      v[u] = idx < total ? plane[idx] : 0;
-    }
+    for (int u = 0; u < 2; ++u) {
+      const int i = base + u * blockDim.x;
+      if (i < total4) {
+        plane[i] = make_int4(0, 0, 0, 0);  // ready for the next spread
+        const int q[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+        int y = (int)fdiv((unsigned)(4 * i), d.ax.by_n), x = 4 * i - y * nx;
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int idx = base + u * blockDim.x;
-      if (idx < total) {
-        plane[idx] = 0;  // ready for the next spread
-        const int y = (int)fdiv((unsigned)idx, d.ax.by_n), x = idx - y * nx;
-        float *slot = reinterpret_cast<float *>(&buf[(y >> 1) * rowp + s_rev[x]]);
-        slot[y & 1] = (float)v[u] * kInvGridScale;
+        for (int e = 0; e < 4; ++e) {
+          float *slot = reinterpret_cast<float *>(&buf[(y >> 1) * rowp + s_rev[x]]);
+          slot[y & 1] = (float)q[e] * kInvGridScale;
+          if (++x == nx) {
+            x = 0;
+            ++y;
+          }
+        }
       }
     }
   }
   __syncthreads();
-  fft_dit(buf, ny / 2, rowp, 1, d.ax, twx, -1.f);
+  fft_dit<false>(buf, ny / 2, d.by_rows, rowp, 1, d.ax, twx);
   // split the packed rows into the two half spectra, in place
   const int ngrp = (h + 1) / 2 + 1;
   for (int idx = threadIdx.x; idx < (ny / 2) * ngrp; idx += blockDim.x) {
@@ -469,7 +556,7 @@ __global__ void __launch_bounds__(kPlaneThreads) plane_fwd_kernel(const __grid_c
       b[nxc + h] = make_float2(Z.y, 0.f);
     } else {
       const int k1 = g, k2 = h - 1 - g;
-      const float2 Z1 = b[k1], M1 = b[(nx - k1) % nx];
+      const float2 Z1 = b[k1], M1 = b[k1 ? nx - k1 : 0];
       const float2 Z2 = b[k2], M2 = b[nx - k2];
       const float2 A1 = make_float2(0.5f * (Z1.x + M1.x), 0.5f * (Z1.y - M1.y));
       const float2 B1 = make_float2(0.5f * (Z1.y + M1.y), -0.5f * (Z1.x - M1.x));
@@ -486,7 +573,7 @@ __global__ void __launch_bounds__(kPlaneThreads) plane_fwd_kernel(const __grid_c
   __syncthreads();
   // the in-place split leaves row y at y*nxc (rowp = 2 nxc: row 2r+1 starts
   // right after row 2r); in global memory rows have the even pitch nxcp
-  fft_dif(buf, nxc, 1, nxc, d.ay, twy, -1.f);
+  fft_dif<false>(buf, nxc, d.ax.by_nxc, 1, nxc, d.ay, twy);
   float2 *out = cgrid + (size_t)z * ny * nxcp;
   for (int idx = threadIdx.x; idx < ny * nxcp; idx += blockDim.x) {
     const int y = (int)fdiv((unsigned)idx, d.ax.by_nxcp), kx = idx - y * nxcp;
@@ -494,7 +581,7 @@ __global__ void __launch_bounds__(kPlaneThreads) plane_fwd_kernel(const __grid_c
   }
 }
 
-__global__ void __launch_bounds__(kPlaneThreads) plane_inv_kernel(const __grid_constant__ PmeDims d0,
+__global__ void __launch_bounds__(kPlaneThreadsMax) plane_inv_kernel(const __grid_constant__ PmeDims d0,
                                                                   const float2 *__restrict__ cgrid,
                                                                   float *__restrict__ phi,
                                                                   const float2 *__restrict__ twx,
@@ -514,16 +601,29 @@ __global__ void __launch_bounds__(kPlaneThreads) plane_inv_kernel(const __grid_c
     z = blockIdx.x - A.plane0;
   }
   const PmeDims &d = *dp;
-  __shared__ short s_unrev[256];  // position in the digit-reversed row -> x
+  __shared__ short s_rev[256];  // x -> position in the digit-reversed row
   const int nx = d.nx, ny = d.ny, nxc = d.nxc, nxcp = d.nxcp, rowp = nx + 2, h = nx / 2;
   const float2 *in = cgrid + (size_t)z * ny * nxcp;
-  fill_rev_table(s_unrev, d.ax, true);
-  for (int idx = threadIdx.x; idx < ny * nxc; idx += blockDim.x) {
-    const int y = (int)fdiv((unsigned)idx, d.ax.by_nxc), kx = idx - y * nxc;
-    buf[idx] = in[y * nxcp + kx];
+  fill_rev_table(s_rev, d.ax, false);
+  // four loads in flight per thread before any store
+  for (int base = threadIdx.x; base < ny * nxc; base += 4 * blockDim.x) {
+    float2 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int idx = base + u * blockDim.x;
+      if (idx < ny * nxc) {
+        const int y = (int)fdiv((unsigned)idx, d.ax.by_nxc), kx = idx - y * nxc;
+        v[u] = in[y * nxcp + kx];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int idx = base + u * blockDim.x;
+      if (idx < ny * nxc) buf[idx] = v[u];
+    }
   }
   __syncthreads();
-  fft_dit(buf, nxc, 1, nxc, d.ay, twy, 1.f);
+  fft_dit<true>(buf, nxc, d.ax.by_nxc, 1, nxc, d.ay, twy);
   // pack pairs of half spectra into one complex row, in place
   const int ngrp = (h + 1) / 2 + 1;
   for (int idx = threadIdx.x; idx < (ny / 2) * ngrp; idx += blockDim.x) {
@@ -544,12 +644,12 @@ __global__ void __launch_bounds__(kPlaneThreads) plane_inv_kernel(const __grid_c
     }
   }
   __syncthreads();
-  fft_dif(buf, ny / 2, rowp, 1, d.ax, twx, 1.f);
+  fft_dif<true>(buf, ny / 2, d.by_rows, rowp, 1, d.ax, twx);
+  // natural order out: consecutive threads write consecutive points
   float *out = phi + (size_t)z * nx * ny;
   for (int idx = threadIdx.x; idx < (ny / 2) * nx; idx += blockDim.x) {
-    const int r = (int)fdiv((unsigned)idx, d.ax.by_n), p = idx - r * nx;
-    const int x = s_unrev[p];
-    const float2 v = buf[r * rowp + p];
+    const int r = (int)fdiv((unsigned)idx, d.ax.by_n), x = idx - r * nx;
+    const float2 v = buf[r * rowp + s_rev[x]];
     out[(2 * r) * nx + x] = v.x;
     out[(2 * r + 1) * nx + x] = v.y;
   }
@@ -570,9 +670,10 @@ __global__ void __launch_bounds__(kPencilThreads) pencil_kernel(const __grid_con
                                                                 const __grid_constant__ CUtensorMap tmap,
                                                                 unsigned *__restrict__ err,
                                                                 const double4 *__restrict__ dbox = nullptr) {
-  // TMA: the slab of 16 complex columns x nz arrives in (and leaves from)
+  // TMA: the slab of ptx complex columns x nz arrives in (and leaves from)
   // buf as one tiled copy of the padded complex grid
-  __shared__ __align__(128) float2 buf[256 * kPencilTX];
+  extern __shared__ float2 dyn[];
+  float2 *const buf = dyn + ((128u - (smem_u32(dyn) & 127u)) & 127u) / sizeof(float2);
   __shared__ __align__(8) unsigned long long s_bar;
   __shared__ short s_unrev_z[256];
   __shared__ double sh_e[kPencilThreads / 32];
@@ -599,13 +700,13 @@ __global__ void __launch_bounds__(kPencilThreads) pencil_kernel(const __grid_con
     Ly = (float)b.y;
     Lz = (float)b.z;
   }
-  const int tiles_x = (nxc + kPencilTX - 1) / kPencilTX;
-  const int py = blk / tiles_x, x0 = (blk - py * tiles_x) * kPencilTX;
+  const int TX = d.ptx, tiles_x = d.ptiles;
+  const int py = blk / tiles_x, x0 = (blk - py * tiles_x) * TX;
   if (TMA) {
     if (threadIdx.x == 0) mbar_init(&s_bar, 1);
     __syncthreads();
     if (threadIdx.x == 0) {
-      mbar_expect_tx(&s_bar, (unsigned)(nz * kPencilTX * sizeof(float2)));
+      mbar_expect_tx(&s_bar, (unsigned)(nz * TX * sizeof(float2)));
       tma_load_3d(buf, &tmap, 2 * x0, py, 0, &s_bar);
     }
     fill_rev_table(s_unrev_z, d.az, true);
@@ -619,13 +720,13 @@ __global__ void __launch_bounds__(kPencilThreads) pencil_kernel(const __grid_con
     }
   } else {
     fill_rev_table(s_unrev_z, d.az, true);
-    for (int idx = threadIdx.x; idx < nz * kPencilTX; idx += blockDim.x) {
-      const int zz = idx / kPencilTX, xt = idx - zz * kPencilTX, kx = x0 + xt;
+    for (int idx = threadIdx.x; idx < nz * TX; idx += blockDim.x) {
+      const int zz = (int)fdiv((unsigned)idx, d.by_ptx), xt = idx - zz * TX, kx = x0 + xt;
       buf[idx] = kx < nxc ? cgrid[((size_t)zz * ny + py) * d.nxcp + kx] : make_float2(0.f, 0.f);
     }
   }
   __syncthreads();
-  fft_dif(buf, kPencilTX, 1, kPencilTX, d.az, twz, -1.f);
+  fft_dif<false>(buf, TX, d.by_ptx, 1, TX, d.az, twz);
   const int ky = dig_unrev(py, d.ay);
   const int nf1 = nx / 2 + (nx & 1), nf2 = ny / 2 + (ny & 1), nf3 = nz / 2 + (nz & 1);
   const FT m2 = (FT)(ky >= nf2 ? ky - ny : ky) / (FT)Ly;
@@ -637,44 +738,44 @@ __global__ void __launch_bounds__(kPencilThreads) pencil_kernel(const __grid_con
   const FT pyv = pf[nx + ky];
   double e = 0.0;
   double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  for (int idx = threadIdx.x; idx < nz * kPencilTX; idx += blockDim.x) {
-    const int pz = idx / kPencilTX, xt = idx - pz * kPencilTX, kx = x0 + xt;
+  for (int idx = threadIdx.x; idx < nz * TX; idx += blockDim.x) {
+    const int pz = (int)fdiv((unsigned)idx, d.by_ptx), xt = idx - pz * TX, kx = x0 + xt;
     if (kx >= nxc) continue;
     const int kz = s_unrev_z[pz];
     FT eterm = 0;
     const FT m1 = (FT)(kx >= nf1 ? kx - nx : kx) / (FT)Lx;
     const FT m3 = (FT)(kz >= nf3 ? kz - nz : kz) / (FT)Lz;
-    const FT msq = m1 * m1 + m2 * m2 + m3 * m3;
+    const FT msq = fma(m1, m1, fma(m2, m2, m3 * m3));
     if (kx != 0 || ky != 0 || kz != 0)
       eterm = exp(-fac * msq) * piv_inv * pf[kx] * pyv * pf[nx + ny + kz] / msq;
     const float2 q = buf[idx];
     if (ENERGY) {
       const FT mult = kx >= 1 ? (FT)2 : (FT)1;
-      const FT t1 = mult * eterm * ((FT)q.x * q.x + (FT)q.y * q.y);
+      const FT t1 = mult * eterm * fma((FT)q.x, (FT)q.x, (FT)q.y * (FT)q.y);
       e += (double)t1;
       if (VIRIAL && eterm != (FT)0) {
         // reference scalar_sum (src/CudaPMERecip.cu:770-790): t1 (vterm m_a m_b - delta_ab)
         const FT vt = (FT)2 * (fac + (FT)1 / msq);
-        v[0] += (double)(t1 * (vt * m1 * m1 - (FT)1));
+        v[0] += (double)(t1 * fma(vt * m1, m1, (FT)-1));
         v[1] += (double)(t1 * vt * m1 * m2);
         v[2] += (double)(t1 * vt * m1 * m3);
-        v[3] += (double)(t1 * (vt * m2 * m2 - (FT)1));
+        v[3] += (double)(t1 * fma(vt * m2, m2, (FT)-1));
         v[4] += (double)(t1 * vt * m2 * m3);
-        v[5] += (double)(t1 * (vt * m3 * m3 - (FT)1));
+        v[5] += (double)(t1 * fma(vt * m3, m3, (FT)-1));
       }
     }
     buf[idx] = make_float2((float)(q.x * eterm), (float)(q.y * eterm));
   }
   __syncthreads();
-  fft_dit(buf, kPencilTX, 1, kPencilTX, d.az, twz, 1.f);
+  fft_dit<true>(buf, TX, d.by_ptx, 1, TX, d.az, twz);
   if (TMA) {
     // columns past the grid's padded width are clipped by the copy
     fence_proxy_async_smem();
     __syncthreads();
     if (threadIdx.x == 0) tma_store_3d(&tmap, 2 * x0, py, 0, buf);
   } else {
-    for (int idx = threadIdx.x; idx < nz * kPencilTX; idx += blockDim.x) {
-      const int zz = idx / kPencilTX, xt = idx - zz * kPencilTX, kx = x0 + xt;
+    for (int idx = threadIdx.x; idx < nz * TX; idx += blockDim.x) {
+      const int zz = (int)fdiv((unsigned)idx, d.by_ptx), xt = idx - zz * TX, kx = x0 + xt;
       if (kx < nxc) cgrid[((size_t)zz * ny + py) * d.nxcp + kx] = buf[idx];
     }
   }
@@ -829,7 +930,7 @@ void dalloc(T *&p, size_t n) {
 }  // namespace
 
 // The tensor map of the pencil slabs: the padded complex grid viewed as
-// floats [nz][ny][2 nxcp], a box of 16 complex columns x 1 row x nz planes.
+// floats [nz][ny][2 nxcp], a box of ptx complex columns x 1 row x nz planes.
 // The encoder is the driver's, fetched through the runtime (no link to the
 // driver library).
 bool encode_pencil_map(CUtensorMap *map, float2 *cgrid, const PmeDims &d) {
@@ -850,12 +951,13 @@ bool encode_pencil_map(CUtensorMap *map, float2 *cgrid, const PmeDims &d) {
     else
       cudaGetLastError();
   }
-  // a row at least one box wide, at most 256 planes, rows of 16-byte multiples
-  if (!fn || d.nz > 256 || (d.nxcp & 1) || 2 * d.nxcp < 2 * kPencilTX) return false;
+  // at most 256 planes, rows and slabs of 16-byte multiples; a slab starts at
+  // an even column, 16-byte aligned
+  if (!fn || d.nz > 256 || (d.nxcp & 1) || (d.ptx & 1) || d.nxcp < d.ptx) return false;
   const cuuint64_t dims[3] = {2ull * d.nxcp, (cuuint64_t)d.ny, (cuuint64_t)d.nz};
   const cuuint64_t strides[2] = {2ull * d.nxcp * sizeof(float),
                                  2ull * d.nxcp * d.ny * sizeof(float)};
-  const cuuint32_t box[3] = {2u * kPencilTX, 1u, (cuuint32_t)d.nz};
+  const cuuint32_t box[3] = {2u * d.ptx, 1u, (cuuint32_t)d.nz};
   const cuuint32_t es[3] = {1u, 1u, 1u};
   return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, cgrid, dims, strides, box, es,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -865,6 +967,50 @@ bool encode_pencil_map(CUtensorMap *map, float2 *cgrid, const PmeDims &d) {
 // shared memory of one plane transform: ny/2 packed rows of nx + 2 complex
 static size_t plane_smem_bytes(int nx, int ny) {
   return (size_t)(ny / 2) * (nx + 2) * sizeof(float2);
+}
+
+// threads of a plane transform: one butterfly of about 8 points a thread and
+// stage up to 1,024.  At 64^2 256 threads do every stage in one go (512 left
+// half of them idle); a 216^2 plane has an SM to itself and needs the warps
+// (20 steps of 998,000 atoms: 59.3 ms with 1,024 threads, 59.9 with 512, 61.2
+// with 256).
+static int plane_threads(int nx, int ny) {
+  const int want = nx * ny / 16;
+  return want <= 256 ? 256 : want <= 1024 ? 512 : 1024;
+}
+static size_t pencil_smem_bytes(const PmeDims &d) { return (size_t)d.nz * d.ptx * sizeof(float2) + 128; }
+
+// The z pencils' slabs: about 16 complex columns, an even number (16-byte
+// aligned slabs), chosen so that the last slab of a row is not left nearly
+// empty (nxc = 33 is two slabs of 18, not 16 + 16 + 1)
+static void set_tiles(PmeDims &d) {
+  const int tiles = std::max(1, (d.nxc + 8) / 16);
+  d.ptx = ((d.nxc + tiles - 1) / tiles + 1) & ~1;
+  d.ptiles = (d.nxc + d.ptx - 1) / d.ptx;
+  d.by_ptx = make_fastdiv((unsigned)d.ptx);
+  d.by_rows = make_fastdiv((unsigned)(d.ny / 2));
+}
+
+static void raise_smem_limits() {
+  APO_CUDA(cudaFuncSetAttribute(plane_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                kPlaneSmemMax));
+  APO_CUDA(cudaFuncSetAttribute(plane_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                kPlaneSmemMax));
+  const auto raise = [](auto *k) {
+    APO_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kPencilSmemMax));
+  };
+  raise(pencil_kernel<true, double, true, true>);
+  raise(pencil_kernel<true, double, true, false>);
+  raise(pencil_kernel<true, float, true, true>);
+  raise(pencil_kernel<true, float, true, false>);
+  raise(pencil_kernel<true, double, false, true>);
+  raise(pencil_kernel<true, double, false, false>);
+  raise(pencil_kernel<true, float, false, true>);
+  raise(pencil_kernel<true, float, false, false>);
+  raise(pencil_kernel<false, double, false, true>);
+  raise(pencil_kernel<false, double, false, false>);
+  raise(pencil_kernel<false, float, false, true>);
+  raise(pencil_kernel<false, float, false, false>);
 }
 
 FastDiv make_fastdiv(unsigned d) {
@@ -881,7 +1027,6 @@ void fill_axis_divisors(FftAxis &a) {
   int prod = 1;
   for (int s = 0; s < a.nrad; ++s) {
     prod *= a.radix[s];
-    a.per_line[s] = make_fastdiv((unsigned)(a.n / a.radix[s]));
     a.dif_mr[s] = make_fastdiv((unsigned)(a.n / prod));
   }
   int tail = 1;
@@ -976,6 +1121,7 @@ void Pme::setup(int nx, int ny, int nz, int order, double kappa, double Lx, doub
   m_d.ax = plan_axis(nx);
   m_d.ay = plan_axis(ny);
   m_d.az = plan_axis(nz);
+  set_tiles(m_d);
   const size_t G = (size_t)nx * ny * nz;
   dalloc(qgrid, G);
   dalloc(cgrid, (size_t)nz * ny * m_d.nxcp);
@@ -1003,10 +1149,7 @@ void Pme::setup(int nx, int ny, int nz, int order, double kappa, double Lx, doub
   APO_CUDA(cudaMemcpy(m_prefac_d, pd.data(), pd.size() * sizeof(double), cudaMemcpyHostToDevice));
   static bool attr = false;
   if (!attr) {
-    APO_CUDA(cudaFuncSetAttribute(plane_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  kPlaneSmemMax));
-    APO_CUDA(cudaFuncSetAttribute(plane_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  kPlaneSmemMax));
+    raise_smem_limits();
     attr = true;
   }
 }
@@ -1024,24 +1167,24 @@ void Pme::spread(const float4 *xyzq_s, const int *counts, cudaStream_t s,
 
 void Pme::forward(cudaStream_t s) {
   const size_t sm = plane_smem_bytes(m_d.nx, m_d.ny);
-  plane_fwd_kernel<<<m_d.nz, kPlaneThreads, sm, s>>>(m_d, qgrid, cgrid, m_tw, m_tw + m_d.nx);
+  plane_fwd_kernel<<<m_d.nz, plane_threads(m_d.nx, m_d.ny), sm, s>>>(m_d, qgrid, cgrid, m_tw, m_tw + m_d.nx);
   APO_LAUNCH_CHECK();
 }
 
 void Pme::convolve(long long *energy, bool calc_energy, bool fp64, cudaStream_t s,
                    long long *virial) {
-  const int tiles_x = (m_d.nxc + kPencilTX - 1) / kPencilTX;
-  const int grid = tiles_x * m_d.ny;
+  const int grid = m_d.ptiles * m_d.ny;
+  const size_t sm = pencil_smem_bytes(m_d);
   const float2 *twz = m_tw + m_d.nx + m_d.ny;
   const bool tma = tensor_copies() && m_err;
 #define APO_PENCIL(E, FT, V)                                                                   \
   do {                                                                                         \
     if (tma)                                                                                   \
-      pencil_kernel<E, FT, V, true><<<grid, kPencilThreads, 0, s>>>(                           \
+      pencil_kernel<E, FT, V, true><<<grid, kPencilThreads, sm, s>>>(                           \
           m_d, cgrid, twz, m_prefac, m_prefac_d, energy, virial, nullptr, nullptr, m_tmap, m_err, \
           m_dbox);                                                                             \
     else                                                                                       \
-      pencil_kernel<E, FT, V, false><<<grid, kPencilThreads, 0, s>>>(                          \
+      pencil_kernel<E, FT, V, false><<<grid, kPencilThreads, sm, s>>>(                          \
           m_d, cgrid, twz, m_prefac, m_prefac_d, energy, virial, nullptr, nullptr, m_tmap, m_err, \
           m_dbox);                                                                             \
   } while (0)
@@ -1061,7 +1204,7 @@ void Pme::convolve(long long *energy, bool calc_energy, bool fp64, cudaStream_t 
 
 void Pme::backward(cudaStream_t s) {
   const size_t sm = plane_smem_bytes(m_d.nx, m_d.ny);
-  plane_inv_kernel<<<m_d.nz, kPlaneThreads, sm, s>>>(m_d, cgrid, phi, m_tw, m_tw + m_d.nx);
+  plane_inv_kernel<<<m_d.nz, plane_threads(m_d.nx, m_d.ny), sm, s>>>(m_d, cgrid, phi, m_tw, m_tw + m_d.nx);
   APO_LAUNCH_CHECK();
 }
 
@@ -1123,7 +1266,8 @@ void PmeMulti::setup(const std::vector<PmeSystemSpec> &systems, int order, long 
   std::vector<int> plane_sys, pencil_sys;
   std::vector<float2> tw;
   std::vector<double> pd;
-  m_plane_smem = 0;
+  m_plane_smem = m_pencil_smem = 0;
+  m_plane_threads = 0;
   for (size_t k = 0; k < systems.size(); ++k) {
     const PmeSystemSpec &y = systems[k];
     if (y.nx % 2 || y.ny % 2 || y.nz % 2 || y.nx <= 0 || y.ny <= 0 || y.nz <= 0)
@@ -1152,6 +1296,9 @@ void PmeMulti::setup(const std::vector<PmeSystemSpec> &systems, int order, long 
     A.d.ax = Pme::plan_axis(y.nx);
     A.d.ay = Pme::plan_axis(y.ny);
     A.d.az = Pme::plan_axis(y.nz);
+    set_tiles(A.d);
+    m_pencil_smem = std::max(m_pencil_smem, pencil_smem_bytes(A.d));
+    m_plane_threads = std::max(m_plane_threads, plane_threads(y.nx, y.ny));
     // offsets for now; turned into pointers once the buffers exist
     A.qgrid = reinterpret_cast<int *>(q);
     A.phi = reinterpret_cast<float *>(q);
@@ -1163,7 +1310,7 @@ void PmeMulti::setup(const std::vector<PmeSystemSpec> &systems, int order, long 
     A.virial = A.energy + kNumEnergyTerms;
     A.plane0 = m_planes;
     A.pencil0 = m_pencils;
-    const int tiles_x = (A.d.nxc + kPencilTX - 1) / kPencilTX;
+    const int tiles_x = A.d.ptiles;
     for (int z = 0; z < y.nz; ++z) plane_sys.push_back((int)k);
     for (int b = 0; b < tiles_x * y.ny; ++b) pencil_sys.push_back((int)k);
     m_planes += y.nz;
@@ -1213,10 +1360,7 @@ void PmeMulti::setup(const std::vector<PmeSystemSpec> &systems, int order, long 
   APO_CUDA(cudaMalloc(&m_pencil_sys, pencil_sys.size() * sizeof(int)));
   APO_CUDA(cudaMemcpy(m_pencil_sys, pencil_sys.data(), pencil_sys.size() * sizeof(int),
                       cudaMemcpyHostToDevice));
-  APO_CUDA(cudaFuncSetAttribute(plane_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                kPlaneSmemMax));
-  APO_CUDA(cudaFuncSetAttribute(plane_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                kPlaneSmemMax));
+  raise_smem_limits();
 }
 
 void PmeMulti::compute(const float4 *xyzq_s, const float4 *origin, const int *cl_sys,
@@ -1230,27 +1374,27 @@ void PmeMulti::compute(const float4 *xyzq_s, const float4 *origin, const int *cl
     case 8: spread_kernel<8><<<blocks, 128, 0, s>>>(xyzq_s, counts, d0, nullptr, origin, m_args, cl_sys); break;
   }
   APO_LAUNCH_CHECK();
-  plane_fwd_kernel<<<m_planes, kPlaneThreads, m_plane_smem, s>>>(d0, nullptr, nullptr, nullptr,
+  plane_fwd_kernel<<<m_planes, m_plane_threads, m_plane_smem, s>>>(d0, nullptr, nullptr, nullptr,
                                                                   nullptr, m_args, m_plane_sys);
   APO_LAUNCH_CHECK();
   if (calc_virial) {
     if (fp64)
-      pencil_kernel<true, double, true><<<m_pencils, kPencilThreads, 0, s>>>(d0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, m_args, m_pencil_sys, kNoTensorMap, nullptr);
+      pencil_kernel<true, double, true><<<m_pencils, kPencilThreads, m_pencil_smem, s>>>(d0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, m_args, m_pencil_sys, kNoTensorMap, nullptr);
     else
-      pencil_kernel<true, float, true><<<m_pencils, kPencilThreads, 0, s>>>(d0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, m_args, m_pencil_sys, kNoTensorMap, nullptr);
+      pencil_kernel<true, float, true><<<m_pencils, kPencilThreads, m_pencil_smem, s>>>(d0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, m_args, m_pencil_sys, kNoTensorMap, nullptr);
   } else if (calc_energy) {
     if (fp64)
-      pencil_kernel<true, double><<<m_pencils, kPencilThreads, 0, s>>>(d0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, m_args, m_pencil_sys, kNoTensorMap, nullptr);
+      pencil_kernel<true, double><<<m_pencils, kPencilThreads, m_pencil_smem, s>>>(d0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, m_args, m_pencil_sys, kNoTensorMap, nullptr);
     else
-      pencil_kernel<true, float><<<m_pencils, kPencilThreads, 0, s>>>(d0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, m_args, m_pencil_sys, kNoTensorMap, nullptr);
+      pencil_kernel<true, float><<<m_pencils, kPencilThreads, m_pencil_smem, s>>>(d0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, m_args, m_pencil_sys, kNoTensorMap, nullptr);
   } else {
     if (fp64)
-      pencil_kernel<false, double><<<m_pencils, kPencilThreads, 0, s>>>(d0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, m_args, m_pencil_sys, kNoTensorMap, nullptr);
+      pencil_kernel<false, double><<<m_pencils, kPencilThreads, m_pencil_smem, s>>>(d0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, m_args, m_pencil_sys, kNoTensorMap, nullptr);
     else
-      pencil_kernel<false, float><<<m_pencils, kPencilThreads, 0, s>>>(d0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, m_args, m_pencil_sys, kNoTensorMap, nullptr);
+      pencil_kernel<false, float><<<m_pencils, kPencilThreads, m_pencil_smem, s>>>(d0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, m_args, m_pencil_sys, kNoTensorMap, nullptr);
   }
   APO_LAUNCH_CHECK();
-  plane_inv_kernel<<<m_planes, kPlaneThreads, m_plane_smem, s>>>(d0, nullptr, nullptr, nullptr,
+  plane_inv_kernel<<<m_planes, m_plane_threads, m_plane_smem, s>>>(d0, nullptr, nullptr, nullptr,
                                                                   nullptr, m_args, m_plane_sys);
   APO_LAUNCH_CHECK();
   switch (m_order) {
@@ -1408,10 +1552,7 @@ unsigned char *static_base() {
   if (!b) {
     void *p = nullptr;
     APO_CUDA(cudaGetSymbolAddress(&p, g_pme_static));
-    APO_CUDA(cudaFuncSetAttribute(plane_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  kPlaneSmemMax));
-    APO_CUDA(cudaFuncSetAttribute(plane_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  kPlaneSmemMax));
+    raise_smem_limits();
     b = static_cast<unsigned char *>(p);
     g_static_base[dev].store(b, std::memory_order_release);
   }
@@ -1462,6 +1603,7 @@ void pme_reciprocal_static(const float4 *xyzq, int n, double Lx, double Ly, doub
   d.kappa = (float)kappa;
   if (!fixed_plan_axis(nx, d.ax) || !fixed_plan_axis(ny, d.ay) || !fixed_plan_axis(nz, d.az))
     throw std::invalid_argument("pme_reciprocal_static: grid sizes must factor into 2, 3, 5 and 7");
+  set_tiles(d);
 
   unsigned char *b = static_base();
   long long *acc = reinterpret_cast<long long *>(b + l.energy);
@@ -1491,16 +1633,17 @@ void pme_reciprocal_static(const float4 *xyzq, int n, double Lx, double Ly, doub
   }
   APO_LAUNCH_CHECK();
   const size_t sm = plane_smem_bytes(nx, ny);
-  plane_fwd_kernel<<<nz, kPlaneThreads, sm, s>>>(d, qgrid, cgrid, tw, tw + nx);
+  plane_fwd_kernel<<<nz, plane_threads(nx, ny), sm, s>>>(d, qgrid, cgrid, tw, tw + nx);
   APO_LAUNCH_CHECK();
-  const int pgrid = ((d.nxc + kPencilTX - 1) / kPencilTX) * ny;
+  const int pgrid = d.ptiles * ny;
+  const size_t psm = pencil_smem_bytes(d);
   const float2 *twz = tw + nx + ny;
   if (fp64)
-    pencil_kernel<true, double><<<pgrid, kPencilThreads, 0, s>>>(d, cgrid, twz, prefac, prefac_d, acc, nullptr, nullptr, nullptr, kNoTensorMap, nullptr);
+    pencil_kernel<true, double><<<pgrid, kPencilThreads, psm, s>>>(d, cgrid, twz, prefac, prefac_d, acc, nullptr, nullptr, nullptr, kNoTensorMap, nullptr);
   else
-    pencil_kernel<true, float><<<pgrid, kPencilThreads, 0, s>>>(d, cgrid, twz, prefac, prefac_d, acc, nullptr, nullptr, nullptr, kNoTensorMap, nullptr);
+    pencil_kernel<true, float><<<pgrid, kPencilThreads, psm, s>>>(d, cgrid, twz, prefac, prefac_d, acc, nullptr, nullptr, nullptr, kNoTensorMap, nullptr);
   APO_LAUNCH_CHECK();
-  plane_inv_kernel<<<nz, kPlaneThreads, sm, s>>>(d, cgrid, phi, tw, tw + nx);
+  plane_inv_kernel<<<nz, plane_threads(nx, ny), sm, s>>>(d, cgrid, phi, tw, tw + nx);
   APO_LAUNCH_CHECK();
   switch (order) {
     case 4: gather_kernel<4><<<blocks, 256, 0, s>>>(xyzq, counts, d, phi, grad, stride, nullptr); break;

@@ -10,7 +10,7 @@
 //   spread      int32 fixed-point atomics into the real grid (deterministic)
 //   plane_fwd   one CTA per z-plane: R2C along x (two rows packed into one
 //               complex FFT), C2C along y; the plane lives in shared memory
-//   pencil      one CTA per (y-row, 16 x-columns): FFT along z, multiply by
+//   pencil      one CTA per (y-row, about 16 x-columns): FFT along z, multiply by
 //               the influence function (energy/virial reduced on the way),
 //               inverse FFT along z
 //   plane_inv   inverse of plane_fwd, writes the real potential grid
@@ -48,10 +48,10 @@ struct FftAxis {
   int n;
   int nrad;
   int radix[8];
-  // per stage s: n / radix[s], and the sub-block length over the radix of
-  // the decimation-in-frequency (n / radix[0..s]) and the decimation-in-time
+  // per stage s: the sub-block length over the radix of the
+  // decimation-in-frequency (n / radix[0..s]) and the decimation-in-time
   // (radix[s+1..]) passes
-  FastDiv per_line[8], dif_mr[8], dit_mr[8];
+  FastDiv dif_mr[8], dit_mr[8];
   FastDiv by_n;      // x / n
   FastDiv by_nxc;    // x / (n/2 + 1)
   FastDiv by_nxcp;   // x / the even pitch of n/2 + 1
@@ -69,6 +69,10 @@ struct PmeDims {
   double rLx, rLy, rLz;   // 1 / box, for the FP64 grid anchoring
   float kappa;
   FftAxis ax, ay, az;
+  // z pencils: complex columns of a slab, slabs of a row
+  int ptx, ptiles;
+  FastDiv by_ptx;         // x / ptx
+  FastDiv by_rows;        // x / (ny / 2), the packed rows of a plane
 };
 
 // One system of a multi-system PME: its grid dimensions and its slices of
@@ -181,7 +185,8 @@ class PmeMulti {
   PmeSysArgs *m_args = nullptr;
   int *m_plane_sys = nullptr, *m_pencil_sys = nullptr;
   int m_planes = 0, m_pencils = 0, m_order = 4, m_max_slots = 0;
-  size_t m_plane_smem = 0;
+  size_t m_plane_smem = 0, m_pencil_smem = 0;
+  int m_plane_threads = 0;
   int *m_q = nullptr;
   float2 *m_c = nullptr;
   float *m_phi = nullptr;
