@@ -43,7 +43,11 @@ NbSetup make_nb_setup(double Lx, double Ly, double Lz, double kappa, double roff
   double roff6 = roff3 * roff3, ron6 = ron3 * ron3;
   s.roffinv3 = (float)(1.0 / roff3);
   s.roffinv6 = (float)(1.0 / roff6);
+  s.kp = (float)(0.365 * kappa);
+  s.sw6 = s.sw12 = 0.f;
   if (ron < roff) {
+    s.sw6 = (float)(1.0 / (roff3 - ron3));
+    s.sw12 = (float)(1.0 / (roff6 - ron6));
     s.k6 = (float)(roff3 / (roff3 - ron3));
     s.k12 = (float)(roff6 / (roff6 - ron6));
     s.dv6 = (float)(-1.0 / (ron3 * roff3));
@@ -80,8 +84,13 @@ __global__ void __launch_bounds__(kThreads) nb_kernel(NbArgs a) {
   // ntype^2 slice per warp, reloaded when the warp's system changes
   const int tab_off = MULTI ? wib * kMaxMultiTypes * kMaxMultiTypes : 0;
   int cur_sys = -1;
+  // the packed pair function takes the second coefficient negated
+  const float vsign = PER_PAIR ? 1.f : -1.f;
   if (!MULTI) {
-    for (int k = threadIdx.x; k < T * T; k += blockDim.x) sh_vdw[k] = a.vdw[k];
+    for (int k = threadIdx.x; k < T * T; k += blockDim.x) {
+      const float2 c = a.vdw[k];
+      sh_vdw[k] = make_float2(c.x, vsign * c.y);
+    }
     __syncthreads();
   }
   const unsigned lt_mask = (1u << lane) - 1u;
@@ -114,7 +123,10 @@ __global__ void __launch_bounds__(kThreads) nb_kernel(NbArgs a) {
     if (MULTI && wk.w != cur_sys) {  // warp-uniform
       __syncwarp();
       T = st.ntype;
-      for (int k = lane; k < T * T; k += 32) sh_vdw[tab_off + k] = a.vdw[st.vdw_off + k];
+      for (int k = lane; k < T * T; k += 32) {
+        const float2 c = a.vdw[st.vdw_off + k];
+        sh_vdw[tab_off + k] = make_float2(c.x, vsign * c.y);
+      }
       __syncwarp();
       cur_sys = wk.w;
     }
@@ -122,7 +134,7 @@ __global__ void __launch_bounds__(kThreads) nb_kernel(NbArgs a) {
     const int islot = wk.x * kTile + lane;
     const float4 xi = a.xyzq_s[islot];
     const bool ivalid = a.perm[islot] >= 0;
-    const float qi = xi.w * (float)kCcelec;
+    const float qi = (PER_PAIR ? 1.f : -1.f) * xi.w * (float)kCcelec;
     // this lane's row of the LJ table
     const float2 *vrow = sh_vdw + tab_off + a.type_s[islot] * T;
     // box around the current positions of the i-cluster

@@ -16,6 +16,8 @@ struct NbSetup {
   float kappa, kappa2, two_kappa_sqrtpi;
   float ewald_e2;             // -kappa^2 log2(e): exp(-kappa^2 r^2) = 2^(ewald_e2 r^2)
   float k6, k12, dv6, dv12, roffinv3, roffinv6;
+  float sw6, sw12;            // k6 / roff^3, k12 / roff^6 (0 without a switching range)
+  float kp;                   // 0.365 kappa, of the erfc approximation's argument
   // LJ tables of this system (multi-system launches): ntype x ntype entries
   // at vdw + vdw_off (and vdw14 + vdw14_off for the 1-4 pairs)
   int vdw_off = 0, vdw14_off = 0, ntype = 0;

@@ -110,15 +110,20 @@ __device__ __forceinline__ void retire_warp(int *sched, int lane) {
   }
 }
 
+// The force switch without a test: with ron < r the inner factors of the
+// Lennard-Jones force are k6 (1/r^3 - 1/roff^3) and k12 (1/r^6 - 1/roff^6),
+// below it 1/r^3 and 1/r^6.  The two forms meet at ron and their ratio falls
+// with r, so the factor in force is always the smaller one (sw6 = k6 / roff^3
+// and sw12 = k12 / roff^6; 0 and k = 1 without a switching range).
+
 // One pair: erfc-Ewald (src/CudaDirectForceKernels.cu:479-489) plus VDW_VFSW
 // (src/CudaDirectForceKernels.cu:263-286).  Returns f with gradient on i =
 // f (x_i - x_j); `in` = inside the cutoff and not excluded, anything else
-// gives 0 (r2raw may then be anything finite, including 0).  With ENERGY the
-// two energies of the pair are added to e_el / e_vdw.
+// gives 0 (whatever r2 then is).  With ENERGY the two energies of the pair
+// are added to e_el / e_vdw.
 template <bool ENERGY>
-__device__ __forceinline__ float pair_force(const NbSetup &st, float r2raw, bool in, float qi,
+__device__ __forceinline__ float pair_force(const NbSetup &st, float r2, bool in, float qi,
                                             float qj, float2 cc, double &e_el, double &e_vdw) {
-  const float r2 = in ? r2raw : 1.f;
   const float rinv = rsqrt_approx(r2);  // r2 >= 1e-2 inside the cutoff: never denormal
   const float rr = r2 * rinv;
   const float rinv2 = rinv * rinv;
@@ -128,16 +133,16 @@ __device__ __forceinline__ float pair_force(const NbSetup &st, float r2raw, bool
   const float el = qq * erfc_v * rinv;
   const float fr_el = fmaf(-qq * st.two_kappa_sqrtpi, exp_v, -el);
   const float rinv3 = rinv * rinv2, rinv6 = rinv3 * rinv3;
-  const bool sw = r2 > st.ron2;
-  const float A6 = sw ? st.k6 : 1.f, B6 = sw ? st.roffinv3 : 0.f;
-  const float A12 = sw ? st.k12 : 1.f, B12 = sw ? st.roffinv6 : 0.f;
-  const float t6 = rinv3 - B6, t12 = rinv6 - B12;
-  const float fr_vdw = (cc.x * A6) * t6 * rinv3 - (cc.y * A12) * t12 * rinv6;
+  const float g6 = fminf(rinv3, fmaf(st.k6, rinv3, -st.sw6));
+  const float g12 = fminf(rinv6, fmaf(st.k12, rinv6, -st.sw12));
+  const float fr_vdw = (cc.x * g6) * rinv3 - (cc.y * g12) * rinv6;
   if (ENERGY && in) {
+    const bool sw = r2 > st.ron2;
+    const float t6 = sw ? rinv3 - st.roffinv3 : rinv3, t12 = sw ? rinv6 - st.roffinv6 : rinv6;
     const float C6 = sw ? 0.f : st.dv6, C12 = sw ? 0.f : st.dv12;
     e_el += (double)el;
-    e_vdw += (double)((1.f / 12.f) * cc.y * (A12 * t12 * t12 + C12) -
-                      (1.f / 6.f) * cc.x * (A6 * t6 * t6 + C6));
+    e_vdw += (double)((1.f / 12.f) * cc.y * (g12 * t12 + C12) -
+                      (1.f / 6.f) * cc.x * (g6 * t6 + C6));
   }
   return in ? (fr_vdw + fr_el) * rinv2 : 0.f;
 }
@@ -187,24 +192,22 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
 }
 
 // pair_force for two j-atoms of one i-atom at once (halves lo and hi), on
-// packed arithmetic: the same terms, with the electrostatic part summed as
-// s = qq (2 kappa / sqrt(pi)) exp + el and subtracted at the end, which is
-// the scalar form's fma(-qq 2 kappa / sqrt(pi), exp, -el) negated (IEEE
-// rounding is symmetric, so that part is bit for bit the same).  Returns
-// the two values f with gradient on i = f (x_i - x_j); a half that is not
-// `in` gives 0 (its r2raw may be anything finite).
+// packed arithmetic.  To spend no instruction on signs, nqq holds -q_i q_j
+// ccelec and the second Lennard-Jones coefficient comes negated (-12 c12);
+// the electrostatic part is nqq exp(-kappa^2 r^2) (t P(t) / r + 2 kappa /
+// sqrt(pi)) with t P(t) exp(-kappa^2 r^2) = erfc(kappa r).  Bound by
+// instruction issue: 37 packed operations and 14 others for two pairs, where
+// selecting the switch's constants and masking the distances took about 15
+// more (40 steps of 24,000 atoms 6.97 -> 6.76 ms, 20 steps of 998,000 65.6 ->
+// 62.6).  Returns the two values f with gradient on i = f (x_i - x_j); a half that is not `in` gives 0.
 template <bool ENERGY>
-__device__ __forceinline__ F2 pair_force2(const NbSetup &st, F2 r2raw, bool in0, bool in1, F2 qq,
+__device__ __forceinline__ F2 pair_force2(const NbSetup &st, F2 r2, bool in0, bool in1, F2 nqq,
                                           float2 cc0, float2 cc1, double &e_el,
                                           double &e_vdw) {
-  const float r2a = in0 ? f2lo(r2raw) : 1.f, r2b = in1 ? f2hi(r2raw) : 1.f;
-  const F2 r2 = f2(r2a, r2b);
-  const F2 rinv = f2(rsqrt_approx(r2a), rsqrt_approx(r2b));
-  const F2 rr = r2 * rinv;
-  const F2 rinv2 = rinv * rinv;
+  const F2 rinv = f2(rsqrt_approx(f2lo(r2)), rsqrt_approx(f2hi(r2)));
+  const F2 den = fma2(f2(st.kp), r2 * rinv, f2(1.f));
   const F2 arg = f2(st.ewald_e2) * r2;
   const F2 ex = f2(ex2_approx(f2lo(arg)), ex2_approx(f2hi(arg)));
-  const F2 den = fma2(f2(0.365f), f2(st.kappa) * rr, f2(1.f));
   const F2 t = f2(rcp_approx(f2lo(den)), rcp_approx(f2hi(den)));
   F2 p = f2(6.816177070e-02f);
   p = fma2(p, t, f2(-3.500733972e-01f));
@@ -215,33 +218,36 @@ __device__ __forceinline__ F2 pair_force2(const NbSetup &st, F2 r2raw, bool in0,
   p = fma2(p, t, f2(2.160071135e-01f));
   p = fma2(p, t, f2(2.028342783e-01f));
   p = fma2(p, t, f2(2.061051130e-01f));
-  const F2 erfc_v = ex * t * p;
-  const F2 el = qq * erfc_v * rinv;
-  const F2 s_el = fma2(qq * f2(st.two_kappa_sqrtpi), ex, el);
+  const F2 tp = t * p;
+  const F2 qe = nqq * ex;
+  const F2 w = fma2(tp, rinv, f2(st.two_kappa_sqrtpi));
+  const F2 rinv2 = rinv * rinv;
   const F2 rinv3 = rinv * rinv2, rinv6 = rinv3 * rinv3;
-  const bool swa = r2a > st.ron2, swb = r2b > st.ron2;
-  const F2 A6 = f2(swa ? st.k6 : 1.f, swb ? st.k6 : 1.f);
-  const F2 B6 = f2(swa ? st.roffinv3 : 0.f, swb ? st.roffinv3 : 0.f);
-  const F2 A12 = f2(swa ? st.k12 : 1.f, swb ? st.k12 : 1.f);
-  const F2 B12 = f2(swa ? st.roffinv6 : 0.f, swb ? st.roffinv6 : 0.f);
-  const F2 t6 = rinv3 - B6, t12 = rinv6 - B12;
-  const F2 m6 = f2(cc0.x, cc1.x) * A6 * t6 * rinv3;
-  const F2 m12 = f2(cc0.y, cc1.y) * A12 * t12 * rinv6;
-  const F2 f = (m6 - m12 - s_el) * rinv2;
+  const F2 s6 = fma2(f2(st.k6), rinv3, f2(-st.sw6)), s12 = fma2(f2(st.k12), rinv6, f2(-st.sw12));
+  const F2 g6 = f2(fminf(f2lo(rinv3), f2lo(s6)), fminf(f2hi(rinv3), f2hi(s6)));
+  const F2 g12 = f2(fminf(f2lo(rinv6), f2lo(s12)), fminf(f2hi(rinv6), f2hi(s12)));
+  F2 f = (f2(cc0.x, cc1.x) * g6) * rinv3;
+  f = fma2(f2(cc0.y, cc1.y) * g12, rinv6, f);
+  f = fma2(qe, w, f) * rinv2;
   if (ENERGY) {
+    const F2 nel = qe * tp * rinv;
     if (in0) {
-      const float C6 = swa ? 0.f : st.dv6, C12 = swa ? 0.f : st.dv12;
-      const float t6a = f2lo(t6), t12a = f2lo(t12);
-      e_el += (double)f2lo(el);
-      e_vdw += (double)((1.f / 12.f) * cc0.y * (f2lo(A12) * t12a * t12a + C12) -
-                        (1.f / 6.f) * cc0.x * (f2lo(A6) * t6a * t6a + C6));
+      const bool sw = f2lo(r2) > st.ron2;
+      const float t6 = sw ? f2lo(rinv3) - st.roffinv3 : f2lo(rinv3);
+      const float t12 = sw ? f2lo(rinv6) - st.roffinv6 : f2lo(rinv6);
+      const float C6 = sw ? 0.f : st.dv6, C12 = sw ? 0.f : st.dv12;
+      e_el -= (double)f2lo(nel);
+      e_vdw -= (double)((1.f / 12.f) * cc0.y * (f2lo(g12) * t12 + C12) +
+                        (1.f / 6.f) * cc0.x * (f2lo(g6) * t6 + C6));
     }
     if (in1) {
-      const float C6 = swb ? 0.f : st.dv6, C12 = swb ? 0.f : st.dv12;
-      const float t6b = f2hi(t6), t12b = f2hi(t12);
-      e_el += (double)f2hi(el);
-      e_vdw += (double)((1.f / 12.f) * cc1.y * (f2hi(A12) * t12b * t12b + C12) -
-                        (1.f / 6.f) * cc1.x * (f2hi(A6) * t6b * t6b + C6));
+      const bool sw = f2hi(r2) > st.ron2;
+      const float t6 = sw ? f2hi(rinv3) - st.roffinv3 : f2hi(rinv3);
+      const float t12 = sw ? f2hi(rinv6) - st.roffinv6 : f2hi(rinv6);
+      const float C6 = sw ? 0.f : st.dv6, C12 = sw ? 0.f : st.dv12;
+      e_el -= (double)f2hi(nel);
+      e_vdw -= (double)((1.f / 12.f) * cc1.y * (f2hi(g12) * t12 + C12) +
+                        (1.f / 6.f) * cc1.x * (f2hi(g6) * t6 + C6));
     }
   }
   return f2(in0 ? f2lo(f) : 0.f, in1 ? f2hi(f) : 0.f);
