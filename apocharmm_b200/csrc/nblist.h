@@ -44,6 +44,7 @@ struct NbListDims {
   int tile_cap = 0, work_cap = 0;
   int mask_cap = 0;               // tiles with an exclusion mask
   int tiles_per_work = 8;
+  int split = 1;                  // warps per i-cluster in the tile search
   int sort_cap = 4096;            // max atoms in one column
 };
 
