@@ -291,7 +291,7 @@ __global__ void rescale_dev_kernel(double4 *__restrict__ slot_off,
   slot_off[s] = v;
   xyzq_s[s] = g >= 0 ? make_float4((float)(c.x + v.x), (float)(c.y + v.y), (float)(c.z + v.z),
                                    (float)c.w)
-                     : make_float4(0.f, 0.f, 0.f, 0.f);
+                     : make_float4(kFarAway, kFarAway, kFarAway, 0.f);
 }
 
 // sorted, cluster-local coordinates (runs after every coordinate update)
@@ -301,7 +301,7 @@ __global__ void refresh_kernel(const double4 *__restrict__ coords, const int *__
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= counts[0]) return;
   int g = perm[s];
-  float4 out = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 out = make_float4(kFarAway, kFarAway, kFarAway, 0.f);
   if (g >= 0) {
     const double4 c = coords[g], o = slot_off[s];
     out = make_float4((float)(c.x + o.x), (float)(c.y + o.y), (float)(c.z + o.z), (float)c.w);

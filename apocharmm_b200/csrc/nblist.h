@@ -48,6 +48,10 @@ struct NbListDims {
   int sort_cap = 4096;            // max atoms in one column
 };
 
+// Where padding slots lie (x, y and z in the sorted coordinates): out of reach
+// of every cutoff, with distances whose squares stay finite.
+constexpr float kFarAway = 1e18f;
+
 // A tile's image code and mask index, packed in its second int.
 __host__ __device__ inline int tile_image(int packed) { return packed & 31; }
 __host__ __device__ inline int tile_mask(int packed) { return (packed >> 5) - 1; }  // -1: none
@@ -121,6 +125,7 @@ class NeighborList {
   double4 *slot_off = nullptr;  // image shift - cluster origin, FP64
   float4 *cl_origin = nullptr;  // per cluster
   float4 *xyzq_s = nullptr;     // sorted, cluster-local coordinates + charge
+                                // (padding: kFarAway, charge 0)
   int *type_s = nullptr;        // sorted LJ type
   int2 *tiles = nullptr;        // (j cluster, image code | (mask index + 1) << 5)
   unsigned *masks = nullptr;    // 32 words per masked tile
