@@ -566,6 +566,9 @@ void ForceManager::calcForce(const float4 *d_xyzq, bool calcEnergy, bool calcVir
   if (clear) APO_CUDA(cudaMemsetAsync(m_Force.p, 0, (size_t)3 * m_Stride * sizeof(long long), s));
   if (calcVirial) calcEnergy = true;
   long long *virial = calcVirial ? m_Energy.p + kNumEnergyTerms : nullptr;
+  // without energies no kernel of the evaluation touches the energy slots:
+  // they are cleared beside it instead of before it
+  if (!calcEnergy) APO_CUDA(cudaEventRecord(m_EvFork, s));
   if (m_Multi)
     APO_CUDA(cudaMemsetAsync(m_Energy.p, 0, m_Energy.n * sizeof(long long), s));
   else
@@ -573,7 +576,7 @@ void ForceManager::calcForce(const float4 *d_xyzq, bool calcEnergy, bool calcVir
                              (kNumEnergyTerms + (calcVirial ? 9 : 0)) * sizeof(long long), s));
   m_VirialValid = calcVirial;
   m_EvalMask = m_ComponentMask;
-  APO_CUDA(cudaEventRecord(m_EvFork, s));
+  if (calcEnergy) APO_CUDA(cudaEventRecord(m_EvFork, s));
   if (m_ComponentMask & 2) {
     APO_CUDA(cudaStreamWaitEvent(m_SNb, m_EvFork, 0));
     NbArgs a;
