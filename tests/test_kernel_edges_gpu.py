@@ -1,0 +1,173 @@
+"""GPU kernels at the sizes where their splits, tiles and remainders change,
+against the FP64 oracle or an explicit restatement in numpy."""
+import numpy as np
+import pytest
+
+from apocharmm_b200 import api
+from apocharmm_b200.systems import solvated_chain, water_box
+from parity_util import oracle_for, rel_rms
+
+pytestmark = pytest.mark.gpu
+
+TIMFAC, KBOLTZ = 0.0488882129, 1.987191e-3
+ATMOSP = 1.4584007e-05
+
+
+# every radix (2 to 8) as first and as last stage, half spectra of odd and even
+# length (nx / 2 + 1), one to several pencil slabs, planes of 256, 512 and 1,024
+# threads; orders with and without the shared-memory patch
+@pytest.mark.parametrize("nfft,order", [((16, 18, 20), 4), ((18, 16, 24), 6), ((20, 28, 30), 4),
+                                        ((42, 40, 50), 6), ((50, 56, 36), 8), ((70, 40, 98), 4),
+                                        ((64, 64, 64), 6), ((128, 100, 60), 4),
+                                        ((90, 216, 32), 6), ((216, 180, 48), 4)])
+def test_reciprocal_space_on_many_grids(tmp_path, nfft, order):
+    s = water_box(300, 21.0, seed=9)
+    st = dict(kappa=0.34, nfft=nfft, order=order, ctofnb=8.0, ctonnb=7.0, cutnb=9.0)
+    psf, prm, fm, ctx = api.system_context(s, str(tmp_path), settings=st)
+    fm.setComponentMask(4)
+    ctx.calculateForces(False, True, False)
+    E, G = oracle_for(s, st).evaluate(parts=("recip", "self"))
+    # single-precision grids: 1e-6 of the gradient (5e-7 measured)
+    assert rel_rms(ctx.getForces(), G) < 5e-6
+    assert ctx.getPotentialEnergy() == pytest.approx(E["epot"], rel=1e-6)
+
+
+@pytest.mark.parametrize("order", [4, 6, 8])
+def test_reciprocal_space_of_atoms_far_apart(tmp_path, order):
+    """Clusters whose grid points span more than the shared-memory patch take
+    the points one by one: 20 waters (two clusters) in a 60 A box."""
+    s = water_box(20, 60.0, seed=4, jitter=3.0)
+    st = dict(kappa=0.34, nfft=(60, 64, 56), order=order, ctofnb=8.0, ctonnb=7.0, cutnb=9.0)
+    psf, prm, fm, ctx = api.system_context(s, str(tmp_path), settings=st)
+    fm.setComponentMask(4)
+    ctx.calculateForces(False, True, False)
+    E, G = oracle_for(s, st).evaluate(parts=("recip", "self"))
+    assert rel_rms(ctx.getForces(), G) < 5e-6
+    assert ctx.getPotentialEnergy() == pytest.approx(E["epot"], rel=1e-6)
+
+
+# 1, 10, 11 and 21 waters fill one cluster or just leave it; 128 and 301 give
+# work items whose last queue batch holds 1 to 32 atoms
+@pytest.mark.parametrize("n", [1, 10, 11, 21, 128, 301])
+@pytest.mark.parametrize("ron", [7.0, 8.0])
+def test_direct_space_remainders(tmp_path, n, ron):
+    L = max(18.5, (3 * n / 0.1003) ** (1.0 / 3.0))
+    s = water_box(n, L, seed=n)
+    st = dict(kappa=0.34, nfft=(20, 20, 20), order=4, ctofnb=8.0, ctonnb=ron, cutnb=9.0)
+    psf, prm, fm, ctx = api.system_context(s, str(tmp_path), settings=st)
+    fm.setComponentMask(2)
+    E, G, W = oracle_for(s, st).evaluate(parts=("direct",), virial=True)
+    # single-precision pairs: gradients to 1e-6 (2.3e-6 measured in these sparse
+    # boxes); energies of up to about 20 kcal/mol a pair, each rounded at 6e-8,
+    # cancel to tenths, so 1e-6 kcal/mol a pair; virial terms are some ten times
+    # larger
+    for energy, virial in ((False, False), (True, False), (True, True)):
+        ctx.calculateForces(False, energy, virial)
+        if n > 1:
+            assert rel_rms(ctx.getForces(), G) < 5e-6
+        if energy:
+            assert ctx.getPotentialEnergy() == pytest.approx(E["epot"], rel=1e-6, abs=5e-6)
+        if virial:
+            assert np.abs(ctx.getVirial() - W).max() < 1e-6 * max(20.0, np.abs(W).max())
+
+
+def _flexible(tmp_path, dt, make):
+    s = water_box(216, 19.0, seed=12)
+    st = dict(kappa=0.34, nfft=(20, 20, 20), order=4, ctofnb=8.0, ctonnb=7.0, cutnb=9.0)
+    keep = api.system_context(s, str(tmp_path), settings=st)
+    fm, ctx = keep[2], keep[3]
+    api.relax(ctx, None, iterations=60)
+    ctx.useHolonomicConstraints(False)
+    x = ctx.getCoordinates()
+    v = np.random.default_rng(5).normal(size=x.shape) * np.sqrt(KBOLTZ * 500.0 / s.mass)[:, None]
+    v -= (s.mass[:, None] * v).sum(0) / s.mass.sum()
+    ctx.setVelocities(v)
+    ctx.calculateForces(True, True, True)
+    g, W = ctx.getForces(), ctx.getVirial()
+    it = make(dt)
+    it.setReferenceTemperature(300.0)
+    it.setNoseHooverPistonMass(2.0)   # light: the passes differ by more than rounding
+    it.setCharmmContext(ctx)
+    it.propagate(1)
+    return s, keep, it, x, v, g, W, dt / TIMFAC
+
+
+def test_nose_hoover_step_equals_explicit_passes(tmp_path):
+    """One unconstrained step: the scalar predictor-corrector passes against
+    three explicit passes over the atoms."""
+    s, keep, it, x, v, g, W, h = _flexible(tmp_path, 0.001, api.CudaNoseHooverIntegrator)
+    m = s.mass[:, None]
+    p = h * v + 0.5 * h * h * g / m          # delta_prev from velocities and first forces,
+    p -= (m * p).sum(0) / m.sum()            # without the drift, removed at step 0
+    d = p - h * h * g / m
+    ke_ref = 0.5 * keep[3].getDegreesOfFreedom() * KBOLTZ * 300.0
+
+    def three(u):
+        return ((0.5 * m * (p / h) ** 2).sum() + (0.5 * m * u ** 2).sum() + (0.5 * m * (d / h) ** 2).sum()) / 3.0
+
+    ke, xi, pred = three(v), 0.0, d
+    for k in range(3):
+        f = 2.0 * h * (ke - ke_ref) / 2.0
+        xi = 0.0 + 0.5 * (f + (f if k == 0 else f0))
+        f0 = f if k == 0 else f0             # the previous force starts as the first one
+        u = (p + pred) / (2.0 * h)
+        pred = d - h * h * xi * u
+        ke = three(u)
+    moved = np.abs(pred - d).max()
+    assert moved > 1e-4                       # the thermostat matters in this step
+    # forces evaluated twice differ by 1e-6 relative (list order): h^2 g / m of
+    # a hydrogen at 1e2 kcal/mol/A is 4e-2 A, so 4e-8 A
+    assert np.abs(keep[3].getCoordinates() - (x + pred)).max() < 2e-7
+    assert np.abs(keep[3].getVelocities() - (pred + p) / (2.0 * h)).max() < 2e-7 / h
+
+
+@pytest.mark.parametrize("passes", [1, 2, 3, 4])
+def test_piston_step_equals_explicit_passes(tmp_path, passes):
+    """One unconstrained cubic step without piston friction: box, coordinates
+    and velocities against explicit passes over the atoms."""
+    def make(dt):
+        it = api.CudaLangevinPistonIntegrator(dt)
+        it.setCrystalType(it.CUBIC)
+        it.setLangevinPistonMass([50.0])
+        it.setMaxPredictorCorrectorIterations(passes)
+        return it
+
+    s, keep, it, x, v, g, W, h = _flexible(tmp_path, 0.001, make)
+    fm, ctx = keep[2], keep[3]
+    m = s.mass[:, None]
+    p = h * v + 0.5 * h * h * g / m
+    p -= (m * p).sum(0) / m.sum()   # the drift is removed at step 0
+    d = p - h * h * g / m
+    ke_ref = 0.5 * ctx.getDegreesOfFreedom() * KBOLTZ * 300.0
+    L = s.box[0]
+    V = L ** 3
+    vfac = 1.0 / ATMOSP / V
+
+    def kin(a):
+        return np.einsum("ia,ib->ab", m * a, a) / (h * h)
+
+    dp0 = vfac * (0.5 * (kin(d) + kin(p)) + W) - np.eye(3)
+    static = dp0 - 0.25 * vfac * kin(d)
+    dp = dp0
+    ke = (0.5 * np.trace(kin(p)) + (0.5 * m * v ** 2).sum() + 0.5 * np.trace(kin(d))) / 3.0
+    pred, r = d, x
+    xx = r + d
+    for k in range(passes):
+        delta = (1.0 / 50.0) * (np.trace(dp) / L) * V * h * h * ATMOSP
+        onvel = 0.5 * delta / h
+        pos = L + delta
+        on, half = h * onvel / L, delta / (pos - 0.5 * delta)
+        f = 2.0 * h * (ke - ke_ref) / 2.0
+        f0 = f if k == 0 else f0
+        xi = 0.5 * (f + f0)
+        u = (p + pred) / (2.0 * h)
+        pred = d - (h * h * xi + h * on) * u
+        xx = r + pred + half * 0.5 * (r + xx)
+        dp = static + 0.25 * vfac * kin(pred)
+        ke = (0.5 * np.trace(kin(p)) + (0.5 * m * u ** 2).sum() + 0.5 * np.trace(kin(pred))) / 3.0
+    assert abs(delta) > 1e-5
+    # the virial of the two evaluations differs by 1e-7 of its largest parts
+    # (1e5 kcal/mol), 1e-2 kcal/mol: delta moves by h^2 / (50 L) of it, 5e-9 A
+    assert fm.getBoxDimensions() == pytest.approx([pos] * 3, abs=2e-8)
+    assert np.abs(ctx.getCoordinates() - xx).max() < 2e-7
+    assert np.abs(ctx.getVelocities() - (pred + p) / (2.0 * h)).max() < 2e-7 / h
