@@ -20,8 +20,10 @@ namespace {
 
 constexpr int kPlaneThreadsMax = 1024;
 // dynamic shared memory a plane transform may use: the SM's 227 KB per
-// block less the kernels' static digit-reversal table
+// block less the kernels' static digit-reversal table, and what is left of it
+// beside the twiddles
 constexpr size_t kPlaneSmemMax = 227 * 1024 - 1024;
+constexpr size_t kPlaneSmemTw = kPlaneSmemMax - 512 * sizeof(float2);
 // the tensor-map argument of launches that move their slabs with plain loads
 const CUtensorMap kNoTensorMap{};
 constexpr int kPencilThreads = 256;
@@ -238,7 +240,7 @@ __device__ __forceinline__ void dft(float2 (&x)[R]) {
 
 template <bool INV>
 __device__ __forceinline__ float2 twiddle(const float2 *tw, int idx) {
-  float2 w = __ldg(tw + idx);
+  float2 w = tw[idx];
   if (INV) w.y = -w.y;
   return w;
 }
@@ -295,7 +297,7 @@ __device__ __forceinline__ void stage(int R, float2 *buf, int nl, FastDiv by_nl,
 
 // natural order in, digit-reversed out
 template <bool INV>
-__device__ void fft_dif(float2 *buf, int nl, FastDiv by_nl, int ls, int es, const FftAxis &a,
+__device__ __forceinline__ void fft_dif(float2 *buf, int nl, FastDiv by_nl, int ls, int es, const FftAxis &a,
                         const float2 *tw) {
   int m = a.n;
   for (int s = 0; s < a.nrad; ++s) {
@@ -306,7 +308,7 @@ __device__ void fft_dif(float2 *buf, int nl, FastDiv by_nl, int ls, int es, cons
 }
 // digit-reversed in, natural order out
 template <bool INV>
-__device__ void fft_dit(float2 *buf, int nl, FastDiv by_nl, int ls, int es, const FftAxis &a,
+__device__ __forceinline__ void fft_dit(float2 *buf, int nl, FastDiv by_nl, int ls, int es, const FftAxis &a,
                         const float2 *tw) {
   int m = 1;
   for (int s = a.nrad - 1; s >= 0; --s) {
@@ -605,15 +607,32 @@ __global__ void __launch_bounds__(128) spread_kernel(const float4 *__restrict__ 
 // ------------------------------------------------------------------------
 // plane transforms
 // ------------------------------------------------------------------------
+// The twiddles of a plane's two axes: copied to shared memory by the block
+// (SMTW; the transforms read them at scattered places, each first touch a trip
+// to the L2), or where the plane leaves no room for them, in global memory.
+template <bool SMTW>
+struct Twiddles {
+  const float2 *x, *y;
+  __device__ __forceinline__ Twiddles(const PmeDims &d, const float2 *twx, const float2 *twy,
+                                      float2 *s_tw)
+      : x(SMTW ? s_tw : twx), y(SMTW ? s_tw + 256 : twy) {
+    if (SMTW) {
+      for (int i = threadIdx.x; i < d.nx; i += blockDim.x) s_tw[i] = twx[i];
+      for (int i = threadIdx.x; i < d.ny; i += blockDim.x) s_tw[256 + i] = twy[i];
+    }
+  }
+};
+
 // The grid dimensions are read through a pointer (to the kernel parameter or
 // to the system's entry of the multi-system table), never copied: the FFT
 // stages index their per-stage divisors at run time.
+template <bool SMTW>
 __global__ void __launch_bounds__(kPlaneThreadsMax) plane_fwd_kernel(const __grid_constant__ PmeDims d0, int *__restrict__ qgrid,
                                                                   float2 *__restrict__ cgrid,
                                                                   const float2 *__restrict__ twx,
                                                                   const float2 *__restrict__ twy,
-                                                                  const PmeSysArgs *__restrict__ multi = nullptr,
-                                                                  const int *__restrict__ plane_sys = nullptr) {
+                                                                  const PmeSysArgs *__restrict__ multi,
+                                                                  const int *__restrict__ plane_sys) {
   extern __shared__ float2 buf[];
   int z = blockIdx.x;
   const PmeDims *dp = &d0;
@@ -628,46 +647,48 @@ __global__ void __launch_bounds__(kPlaneThreadsMax) plane_fwd_kernel(const __gri
   }
   const PmeDims &d = *dp;
   __shared__ short s_rev[256];  // x -> position in the digit-reversed row
+  __shared__ float2 s_tw[SMTW ? 512 : 1];
   const int nx = d.nx, ny = d.ny, nxc = d.nxc, nxcp = d.nxcp, rowp = nx + 2, h = nx / 2;
-  // four points a thread and load (nx and ny are even, so a plane is a
-  // multiple of 16 bytes; the four points may run into the next row), two
-  // loads in flight, the first ones while the table is made
-  int4 *plane = reinterpret_cast<int4 *>(qgrid + (size_t)z * nx * ny);
-  const int total4 = nx * ny / 4;
-  int4 v[2];
+  // two neighbouring points of two rows a thread and turn (nx is even, so
+  // pairs are 8-byte aligned), two turns in flight, the first while the
+  // tables are made: a packed row takes both rows' points in one store
+  int *plane = qgrid + (size_t)z * nx * ny;
+  const int total = (ny / 2) * h;
+  int2 v0[2], v1[2];
   const auto fetch = [&](int base) {
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int i = base + u * blockDim.x;
-      if (i < total4) v[u] = plane[i];
+      if (i < total) {
+        const int r = (int)fdiv((unsigned)i, d.by_hx), x = 2 * (i - r * h);
+        v0[u] = *reinterpret_cast<int2 *>(plane + 2 * r * nx + x);
+        v1[u] = *reinterpret_cast<int2 *>(plane + (2 * r + 1) * nx + x);
+      }
     }
   };
   fetch(threadIdx.x);
   fill_rev_table(s_rev, d.ax, false);
+  const Twiddles<SMTW> tw(d, twx, twy, s_tw);
   __syncthreads();
-  for (int base = threadIdx.x; base < total4; base += 2 * blockDim.x) {
+  for (int base = threadIdx.x; base < total; base += 2 * blockDim.x) {
     if (base != (int)threadIdx.x) fetch(base);
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int i = base + u * blockDim.x;
-      if (i < total4) {
-        plane[i] = make_int4(0, 0, 0, 0);  // ready for the next spread
-        const int q[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
-        int y = (int)fdiv((unsigned)(4 * i), d.ax.by_n), x = 4 * i - y * nx;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          float *slot = reinterpret_cast<float *>(&buf[(y >> 1) * rowp + s_rev[x]]);
-          slot[y & 1] = (float)q[e] * kInvGridScale;
-          if (++x == nx) {
-            x = 0;
-            ++y;
-          }
-        }
+      if (i < total) {
+        const int r = (int)fdiv((unsigned)i, d.by_hx), x = 2 * (i - r * h);
+        // ready for the next spread
+        *reinterpret_cast<int2 *>(plane + 2 * r * nx + x) = make_int2(0, 0);
+        *reinterpret_cast<int2 *>(plane + (2 * r + 1) * nx + x) = make_int2(0, 0);
+        buf[r * rowp + s_rev[x]] =
+            make_float2((float)v0[u].x * kInvGridScale, (float)v1[u].x * kInvGridScale);
+        buf[r * rowp + s_rev[x + 1]] =
+            make_float2((float)v0[u].y * kInvGridScale, (float)v1[u].y * kInvGridScale);
       }
     }
   }
   __syncthreads();
-  fft_dit<false>(buf, ny / 2, d.by_rows, rowp, 1, d.ax, twx);
+  fft_dit<false>(buf, ny / 2, d.by_rows, rowp, 1, d.ax, tw.x);
   // split the packed rows into the two half spectra, in place
   const int ngrp = (h + 1) / 2 + 1;
   for (int idx = threadIdx.x; idx < (ny / 2) * ngrp; idx += blockDim.x) {
@@ -696,7 +717,7 @@ __global__ void __launch_bounds__(kPlaneThreadsMax) plane_fwd_kernel(const __gri
   __syncthreads();
   // the in-place split leaves row y at y*nxc (rowp = 2 nxc: row 2r+1 starts
   // right after row 2r); in global memory rows have the even pitch nxcp
-  fft_dif<false>(buf, nxc, d.ax.by_nxc, 1, nxc, d.ay, twy);
+  fft_dif<false>(buf, nxc, d.ax.by_nxc, 1, nxc, d.ay, tw.y);
   float2 *out = cgrid + (size_t)z * ny * nxcp;
   for (int idx = threadIdx.x; idx < ny * nxcp; idx += blockDim.x) {
     const int y = (int)fdiv((unsigned)idx, d.ax.by_nxcp), kx = idx - y * nxcp;
@@ -704,13 +725,14 @@ __global__ void __launch_bounds__(kPlaneThreadsMax) plane_fwd_kernel(const __gri
   }
 }
 
+template <bool SMTW>
 __global__ void __launch_bounds__(kPlaneThreadsMax) plane_inv_kernel(const __grid_constant__ PmeDims d0,
                                                                   const float2 *__restrict__ cgrid,
                                                                   float *__restrict__ phi,
                                                                   const float2 *__restrict__ twx,
                                                                   const float2 *__restrict__ twy,
-                                                                  const PmeSysArgs *__restrict__ multi = nullptr,
-                                                                  const int *__restrict__ plane_sys = nullptr) {
+                                                                  const PmeSysArgs *__restrict__ multi,
+                                                                  const int *__restrict__ plane_sys) {
   extern __shared__ float2 buf[];
   int z = blockIdx.x;
   const PmeDims *dp = &d0;
@@ -725,9 +747,11 @@ __global__ void __launch_bounds__(kPlaneThreadsMax) plane_inv_kernel(const __gri
   }
   const PmeDims &d = *dp;
   __shared__ short s_rev[256];  // x -> position in the digit-reversed row
+  __shared__ float2 s_tw[SMTW ? 512 : 1];
   const int nx = d.nx, ny = d.ny, nxc = d.nxc, nxcp = d.nxcp, rowp = nx + 2, h = nx / 2;
   const float2 *in = cgrid + (size_t)z * ny * nxcp;
   fill_rev_table(s_rev, d.ax, false);
+  const Twiddles<SMTW> tw(d, twx, twy, s_tw);
   // four loads in flight per thread before any store
   for (int base = threadIdx.x; base < ny * nxc; base += 4 * blockDim.x) {
     float2 v[4];
@@ -746,7 +770,7 @@ __global__ void __launch_bounds__(kPlaneThreadsMax) plane_inv_kernel(const __gri
     }
   }
   __syncthreads();
-  fft_dit<true>(buf, nxc, d.ax.by_nxc, 1, nxc, d.ay, twy);
+  fft_dit<true>(buf, nxc, d.ax.by_nxc, 1, nxc, d.ay, tw.y);
   // pack pairs of half spectra into one complex row, in place
   const int ngrp = (h + 1) / 2 + 1;
   for (int idx = threadIdx.x; idx < (ny / 2) * ngrp; idx += blockDim.x) {
@@ -767,14 +791,14 @@ __global__ void __launch_bounds__(kPlaneThreadsMax) plane_inv_kernel(const __gri
     }
   }
   __syncthreads();
-  fft_dif<true>(buf, ny / 2, d.by_rows, rowp, 1, d.ax, twx);
-  // natural order out: consecutive threads write consecutive points
+  fft_dif<true>(buf, ny / 2, d.by_rows, rowp, 1, d.ax, tw.x);
+  // natural order out: consecutive threads write consecutive pairs of points
   float *out = phi + (size_t)z * nx * ny;
-  for (int idx = threadIdx.x; idx < (ny / 2) * nx; idx += blockDim.x) {
-    const int r = (int)fdiv((unsigned)idx, d.ax.by_n), x = idx - r * nx;
-    const float2 v = buf[r * rowp + s_rev[x]];
-    out[(2 * r) * nx + x] = v.x;
-    out[(2 * r + 1) * nx + x] = v.y;
+  for (int i = threadIdx.x; i < (ny / 2) * h; i += blockDim.x) {
+    const int r = (int)fdiv((unsigned)i, d.by_hx), x = 2 * (i - r * h);
+    const float2 a = buf[r * rowp + s_rev[x]], b = buf[r * rowp + s_rev[x + 1]];
+    *reinterpret_cast<float2 *>(out + 2 * r * nx + x) = make_float2(a.x, b.x);
+    *reinterpret_cast<float2 *>(out + (2 * r + 1) * nx + x) = make_float2(a.y, b.y);
   }
 }
 
@@ -799,6 +823,7 @@ __global__ void __launch_bounds__(kPencilThreads) pencil_kernel(const __grid_con
   float2 *const buf = dyn + ((128u - (smem_u32(dyn) & 127u)) & 127u) / sizeof(float2);
   __shared__ __align__(8) unsigned long long s_bar;
   __shared__ short s_unrev_z[256];
+  __shared__ float2 s_tw[256];
   __shared__ double sh_e[kPencilThreads / 32];
   __shared__ double sh_v[6][kPencilThreads / 32];
   int blk = blockIdx.x;
@@ -825,6 +850,7 @@ __global__ void __launch_bounds__(kPencilThreads) pencil_kernel(const __grid_con
   }
   const int TX = d.ptx, tiles_x = d.ptiles;
   const int py = blk / tiles_x, x0 = (blk - py * tiles_x) * TX;
+  for (int i = threadIdx.x; i < nz; i += blockDim.x) s_tw[i] = twz[i];
   if (TMA) {
     if (threadIdx.x == 0) mbar_init(&s_bar, 1);
     __syncthreads();
@@ -849,7 +875,7 @@ __global__ void __launch_bounds__(kPencilThreads) pencil_kernel(const __grid_con
     }
   }
   __syncthreads();
-  fft_dif<false>(buf, TX, d.by_ptx, 1, TX, d.az, twz);
+  fft_dif<false>(buf, TX, d.by_ptx, 1, TX, d.az, s_tw);
   const int ky = dig_unrev(py, d.ay);
   const int nf1 = nx / 2 + (nx & 1), nf2 = ny / 2 + (ny & 1), nf3 = nz / 2 + (nz & 1);
   const FT m2 = (FT)(ky >= nf2 ? ky - ny : ky) / (FT)Ly;
@@ -890,7 +916,7 @@ __global__ void __launch_bounds__(kPencilThreads) pencil_kernel(const __grid_con
     buf[idx] = make_float2((float)(q.x * eterm), (float)(q.y * eterm));
   }
   __syncthreads();
-  fft_dit<true>(buf, TX, d.by_ptx, 1, TX, d.az, twz);
+  fft_dit<true>(buf, TX, d.by_ptx, 1, TX, d.az, s_tw);
   if (TMA) {
     // columns past the grid's padded width are clipped by the copy
     fence_proxy_async_smem();
@@ -1240,13 +1266,18 @@ static void set_tiles(PmeDims &d) {
   d.ptiles = (d.nxc + d.ptx - 1) / d.ptx;
   d.by_ptx = make_fastdiv((unsigned)d.ptx);
   d.by_rows = make_fastdiv((unsigned)(d.ny / 2));
+  d.by_hx = make_fastdiv((unsigned)(d.nx / 2));
 }
 
 static void raise_smem_limits() {
-  APO_CUDA(cudaFuncSetAttribute(plane_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                kPlaneSmemMax));
-  APO_CUDA(cudaFuncSetAttribute(plane_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                kPlaneSmemMax));
+  APO_CUDA(cudaFuncSetAttribute(plane_fwd_kernel<true>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, kPlaneSmemTw));
+  APO_CUDA(cudaFuncSetAttribute(plane_fwd_kernel<false>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, kPlaneSmemMax));
+  APO_CUDA(cudaFuncSetAttribute(plane_inv_kernel<true>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, kPlaneSmemTw));
+  APO_CUDA(cudaFuncSetAttribute(plane_inv_kernel<false>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, kPlaneSmemMax));
   const auto raise = [](auto *k) {
     APO_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kPencilSmemMax));
   };
@@ -1418,7 +1449,8 @@ void Pme::spread(const float4 *xyzq_s, const int *counts, cudaStream_t s,
 
 void Pme::forward(cudaStream_t s) {
   const size_t sm = plane_smem_bytes(m_d.nx, m_d.ny);
-  plane_fwd_kernel<<<m_d.nz, plane_threads(m_d.nx, m_d.ny), sm, s>>>(m_d, qgrid, cgrid, m_tw, m_tw + m_d.nx);
+  (sm <= kPlaneSmemTw ? plane_fwd_kernel<true> : plane_fwd_kernel<false>)<<<m_d.nz, plane_threads(m_d.nx, m_d.ny), sm, s>>>(
+      m_d, qgrid, cgrid, m_tw, m_tw + m_d.nx, nullptr, nullptr);
   APO_LAUNCH_CHECK();
 }
 
@@ -1455,7 +1487,8 @@ void Pme::convolve(long long *energy, bool calc_energy, bool fp64, cudaStream_t 
 
 void Pme::backward(cudaStream_t s) {
   const size_t sm = plane_smem_bytes(m_d.nx, m_d.ny);
-  plane_inv_kernel<<<m_d.nz, plane_threads(m_d.nx, m_d.ny), sm, s>>>(m_d, cgrid, phi, m_tw, m_tw + m_d.nx);
+  (sm <= kPlaneSmemTw ? plane_inv_kernel<true> : plane_inv_kernel<false>)<<<m_d.nz, plane_threads(m_d.nx, m_d.ny), sm, s>>>(
+      m_d, cgrid, phi, m_tw, m_tw + m_d.nx, nullptr, nullptr);
   APO_LAUNCH_CHECK();
 }
 
@@ -1625,7 +1658,7 @@ void PmeMulti::compute(const float4 *xyzq_s, const float4 *origin, const int *cl
     case 8: spread_kernel<8><<<blocks, 128, 0, s>>>(xyzq_s, counts, d0, nullptr, origin, m_args, cl_sys); break;
   }
   APO_LAUNCH_CHECK();
-  plane_fwd_kernel<<<m_planes, m_plane_threads, m_plane_smem, s>>>(d0, nullptr, nullptr, nullptr,
+  (m_plane_smem <= kPlaneSmemTw ? plane_fwd_kernel<true> : plane_fwd_kernel<false>)<<<m_planes, m_plane_threads, m_plane_smem, s>>>(d0, nullptr, nullptr, nullptr,
                                                                   nullptr, m_args, m_plane_sys);
   APO_LAUNCH_CHECK();
   if (calc_virial) {
@@ -1645,7 +1678,7 @@ void PmeMulti::compute(const float4 *xyzq_s, const float4 *origin, const int *cl
       pencil_kernel<false, float><<<m_pencils, kPencilThreads, m_pencil_smem, s>>>(d0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, m_args, m_pencil_sys, kNoTensorMap, nullptr);
   }
   APO_LAUNCH_CHECK();
-  plane_inv_kernel<<<m_planes, m_plane_threads, m_plane_smem, s>>>(d0, nullptr, nullptr, nullptr,
+  (m_plane_smem <= kPlaneSmemTw ? plane_inv_kernel<true> : plane_inv_kernel<false>)<<<m_planes, m_plane_threads, m_plane_smem, s>>>(d0, nullptr, nullptr, nullptr,
                                                                   nullptr, m_args, m_plane_sys);
   APO_LAUNCH_CHECK();
   switch (m_order) {
@@ -1884,7 +1917,8 @@ void pme_reciprocal_static(const float4 *xyzq, int n, double Lx, double Ly, doub
   }
   APO_LAUNCH_CHECK();
   const size_t sm = plane_smem_bytes(nx, ny);
-  plane_fwd_kernel<<<nz, plane_threads(nx, ny), sm, s>>>(d, qgrid, cgrid, tw, tw + nx);
+  (sm <= kPlaneSmemTw ? plane_fwd_kernel<true> : plane_fwd_kernel<false>)<<<nz, plane_threads(nx, ny), sm, s>>>(
+      d, qgrid, cgrid, tw, tw + nx, nullptr, nullptr);
   APO_LAUNCH_CHECK();
   const int pgrid = d.ptiles * ny;
   const size_t psm = pencil_smem_bytes(d);
@@ -1894,7 +1928,8 @@ void pme_reciprocal_static(const float4 *xyzq, int n, double Lx, double Ly, doub
   else
     pencil_kernel<true, float><<<pgrid, kPencilThreads, psm, s>>>(d, cgrid, twz, prefac, prefac_d, acc, nullptr, nullptr, nullptr, kNoTensorMap, nullptr);
   APO_LAUNCH_CHECK();
-  plane_inv_kernel<<<nz, plane_threads(nx, ny), sm, s>>>(d, cgrid, phi, tw, tw + nx);
+  (sm <= kPlaneSmemTw ? plane_inv_kernel<true> : plane_inv_kernel<false>)<<<nz, plane_threads(nx, ny), sm, s>>>(
+      d, cgrid, phi, tw, tw + nx, nullptr, nullptr);
   APO_LAUNCH_CHECK();
   switch (order) {
     case 4: gather_direct_kernel<4><<<blocks, 256, 0, s>>>(xyzq, counts, d, phi, grad, stride, nullptr); break;

@@ -73,6 +73,7 @@ struct PmeDims {
   int ptx, ptiles;
   FastDiv by_ptx;         // x / ptx
   FastDiv by_rows;        // x / (ny / 2), the packed rows of a plane
+  FastDiv by_hx;          // x / (nx / 2)
 };
 
 // One system of a multi-system PME: its grid dimensions and its slices of
