@@ -76,8 +76,11 @@ using namespace nbdetail;
 constexpr int kWarps = 4;
 constexpr int kThreads = kWarps * 32;
 
+// (with energies the packed form is held to 128 registers, four blocks an SM:
+// it took 167 with the virial, three blocks; 40 piston steps of 24,000 atoms
+// 8.86 -> 8.70 ms, an evaluation with virial 603 -> 577 us)
 template <bool ENERGY, bool PER_PAIR, bool VIRIAL = false, bool MULTI = false>
-__global__ void __launch_bounds__(kThreads) nb_kernel(NbArgs a) {
+__global__ void __launch_bounds__(kThreads, ENERGY && !PER_PAIR ? 4 : 1) nb_kernel(NbArgs a) {
   // the j-atoms that pass the box test, compacted: position and charge (for
   // the packed arithmetic as pairs of j-atoms: {x0 x1 y0 y1} and {z0 z1 q0
   // q1}), LJ type, and the list slot (queue) or tile lane (single tile).
