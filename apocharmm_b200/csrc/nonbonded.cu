@@ -839,9 +839,18 @@ void dispatch_q(const NbArgs &a, bool energy, bool per_pair, bool virial, cudaSt
   }
 }
 
+// Lists of up to this many slots leave room on every SM: the persistent grid
+// takes three blocks an SM where four fit, so that the blocks of the
+// reciprocal-space kernels, which cannot fill the GPU on their own at these
+// sizes, run beside it instead of after it (40 steps of 24,000 atoms 5.60 ->
+// 5.05 ms, of 42,000 6.37 -> 5.95, 20 steps of 53,000 5.36 -> 5.12, of 80,000
+// 7.47 -> 7.50, 40 of 107,000 15.35 -> 15.65).  Only without energies: that
+// kernel fills an SM's registers less evenly and loses (8.70 -> 9.08 ms).
+constexpr int kSharedSmSlots = 65536;
+
 template <bool E, bool P, bool V = false, bool M = false>
 void launch_t(const NbArgs &a, cudaStream_t s) {
-  static int grid = 0;
+  static int grid = 0, shared_grid = 0;
   size_t sm = M ? (size_t)kWarps * kMaxMultiTypes * kMaxMultiTypes * sizeof(float2)
                 : (size_t)a.ntype * a.ntype * sizeof(float2);
   if (!grid) {
@@ -853,8 +862,10 @@ void launch_t(const NbArgs &a, cudaStream_t s) {
     APO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, nb_kernel<E, P, V, M>, kThreads,
                                                            64 * 1024 > sm ? sm : 64 * 1024));
     grid = nsm * (per > 0 ? per : 1);
+    shared_grid = !E && per > 3 ? nsm * 3 : grid;
   }
-  nb_kernel<E, P, V, M><<<launch_grid(grid, a), kThreads, sm, s>>>(a);
+  const int resident = a.stride <= kSharedSmSlots ? shared_grid : grid;
+  nb_kernel<E, P, V, M><<<launch_grid(resident, a), kThreads, sm, s>>>(a);
   APO_LAUNCH_CHECK();
 }
 
