@@ -76,11 +76,8 @@ using namespace nbdetail;
 constexpr int kWarps = 4;
 constexpr int kThreads = kWarps * 32;
 
-// (with energies the packed form is held to 128 registers, four blocks an SM:
-// it took 167 with the virial, three blocks; 40 piston steps of 24,000 atoms
-// 8.86 -> 8.70 ms, an evaluation with virial 603 -> 577 us)
-template <bool ENERGY, bool PER_PAIR, bool VIRIAL = false, bool MULTI = false>
-__global__ void __launch_bounds__(kThreads, ENERGY && !PER_PAIR ? 4 : 1) nb_kernel(NbArgs a) {
+template <bool ENERGY, bool PER_PAIR, bool VIRIAL, bool MULTI>
+__device__ __forceinline__ void nb_body(const NbArgs &a) {
   // the j-atoms that pass the box test, compacted: position and charge (for
   // the packed arithmetic as pairs of j-atoms: {x0 x1 y0 y1} and {z0 z1 q0
   // q1}), LJ type, and the list slot (queue) or tile lane (single tile).
@@ -476,6 +473,19 @@ __global__ void __launch_bounds__(kThreads, ENERGY && !PER_PAIR ? 4 : 1) nb_kern
   }
 }
 
+template <bool ENERGY, bool PER_PAIR, bool VIRIAL, bool MULTI>
+__global__ void __launch_bounds__(kThreads) nb_kernel(NbArgs a) {
+  nb_body<ENERGY, PER_PAIR, VIRIAL, MULTI>(a);
+}
+// with energies the packed form is held to 128 registers, four blocks an SM: it
+// took 167 with the virial, three blocks (40 piston steps of 24,000 atoms 8.86
+// -> 8.70 ms, an evaluation with virial 603 -> 577 us).  Without energies the
+// compiler's own 122 (four blocks) stand.
+template <bool ENERGY, bool PER_PAIR, bool VIRIAL, bool MULTI>
+__global__ void __launch_bounds__(kThreads, 4) nb_energy_kernel(NbArgs a) {
+  nb_body<ENERGY, PER_PAIR, VIRIAL, MULTI>(a);
+}
+
 // ---------------------------------------------------------------------------
 // Grouped-queue variant.  The i-cluster is split into four 8-atom groups
 // (the neighbour list orders each cluster as two z-halves of two x-halves,
@@ -850,6 +860,9 @@ constexpr int kSharedSmSlots = 65536;
 
 template <bool E, bool P, bool V = false, bool M = false>
 void launch_t(const NbArgs &a, cudaStream_t s) {
+  void (*kernel)(NbArgs);
+  if constexpr (E && !P) kernel = nb_energy_kernel<E, P, V, M>;
+  else kernel = nb_kernel<E, P, V, M>;
   static int grid = 0, shared_grid = 0;
   size_t sm = M ? (size_t)kWarps * kMaxMultiTypes * kMaxMultiTypes * sizeof(float2)
                 : (size_t)a.ntype * a.ntype * sizeof(float2);
@@ -857,15 +870,15 @@ void launch_t(const NbArgs &a, cudaStream_t s) {
     int dev, nsm, per = 0;
     APO_CUDA(cudaGetDevice(&dev));
     APO_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    APO_CUDA(cudaFuncSetAttribute(nb_kernel<E, P, V, M>,
+    APO_CUDA(cudaFuncSetAttribute(kernel,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
-    APO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, nb_kernel<E, P, V, M>, kThreads,
+    APO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, kThreads,
                                                            64 * 1024 > sm ? sm : 64 * 1024));
     grid = nsm * (per > 0 ? per : 1);
     shared_grid = !E && per > 3 ? nsm * 3 : grid;
   }
   const int resident = a.stride <= kSharedSmSlots ? shared_grid : grid;
-  nb_kernel<E, P, V, M><<<launch_grid(resident, a), kThreads, sm, s>>>(a);
+  kernel<<<launch_grid(resident, a), kThreads, sm, s>>>(a);
   APO_LAUNCH_CHECK();
 }
 
