@@ -1344,7 +1344,7 @@ void CudaIntegrator::setNonbondedListUpdateFrequency(int f) {
 
 cudaStream_t CudaIntegrator::stream() const { return m_Ctx ? m_Ctx->stream() : nullptr; }
 
-int CudaIntegrator::kernelsPerRebuild() const { return 11; }
+int CudaIntegrator::kernelsPerRebuild() const { return 9; }
 
 void CudaIntegrator::setCharmmContext(std::shared_ptr<CharmmContext> ctx) {
   if (m_Ctx) throw std::invalid_argument("A CharmmContext object was already set for this CudaIntegrator.");

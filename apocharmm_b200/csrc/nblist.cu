@@ -223,13 +223,18 @@ __global__ void col_sort_kernel(int ncol, const int *__restrict__ col_count,
   }
 }
 
-// (4b) cluster origins, one warp per cluster: the centre of the wrapped
+// (5) cluster origins, sorted coordinates and bounding boxes, one warp per
+// cluster: the centre of the wrapped
 // positions rounded to a multiple of 1/64 A (exact in single precision for
-// any box below 2^17 A), and per slot the FP64 offset image shift - origin
-__global__ void origin_kernel(const float4 *__restrict__ xyzq, const int *__restrict__ perm,
+// any box below 2^17 A), per slot the FP64 offset image shift - origin and
+// the cluster-local coordinates of the FP64 state, and the box around them
+// (one launch instead of three on the way of every rebuild)
+__global__ void cluster_kernel(const float4 *__restrict__ xyzq, const int *__restrict__ perm,
                               const float4 *__restrict__ slot_shift,
                               const NbSysDims *__restrict__ sysd, const int *__restrict__ cl_sys,
                               float4 *__restrict__ cl_origin, double4 *__restrict__ slot_off,
+                              const double4 *__restrict__ coords, float4 *__restrict__ xyzq_s,
+                              float4 *__restrict__ bb_c, float4 *__restrict__ bb_h,
                               const int *__restrict__ counts) {
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -238,8 +243,12 @@ __global__ void origin_kernel(const float4 *__restrict__ xyzq, const int *__rest
   const int s = w * kTile + lane;
   const int g = perm[s];
   float4 p = make_float4(0.f, 0.f, 0.f, 0.f), sh = slot_shift[s];
-  if (g >= 0) p = xyzq[g];
   const bool valid = g >= 0;
+  double4 c = make_double4(0.0, 0.0, 0.0, 0.0);
+  if (valid) {
+    p = xyzq[g];
+    c = coords[g];
+  }
   float mnx = valid ? p.x + sh.x : INFINITY, mny = valid ? p.y + sh.y : INFINITY,
         mnz = valid ? p.z + sh.z : INFINITY;
   float mxx = valid ? p.x + sh.x : -INFINITY, mxy = valid ? p.y + sh.y : -INFINITY,
@@ -263,8 +272,29 @@ __global__ void origin_kernel(const float4 *__restrict__ xyzq, const int *__rest
   // the wrap shift is k * L with a small integer k
   const double kx = rint((double)sh.x / (double)d.Lx), ky = rint((double)sh.y / (double)d.Ly),
                kz = rint((double)sh.z / (double)d.Lz);
-  slot_off[s] = make_double4(kx * d.Lxd - (double)ox, ky * d.Lyd - (double)oy,
-                             kz * d.Lzd - (double)oz, 0.0);
+  const double4 off = make_double4(kx * d.Lxd - (double)ox, ky * d.Lyd - (double)oy,
+                                   kz * d.Lzd - (double)oz, 0.0);
+  slot_off[s] = off;
+  const float4 q = valid ? make_float4((float)(c.x + off.x), (float)(c.y + off.y),
+                                       (float)(c.z + off.z), (float)c.w)
+                         : make_float4(kFarAway, kFarAway, kFarAway, 0.f);
+  xyzq_s[s] = q;
+  mnx = valid ? q.x : INFINITY, mny = valid ? q.y : INFINITY, mnz = valid ? q.z : INFINITY;
+  mxx = valid ? q.x : -INFINITY, mxy = valid ? q.y : -INFINITY, mxz = valid ? q.z : -INFINITY;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    mnx = fminf(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
+    mny = fminf(mny, __shfl_xor_sync(0xffffffffu, mny, o));
+    mnz = fminf(mnz, __shfl_xor_sync(0xffffffffu, mnz, o));
+    mxx = fmaxf(mxx, __shfl_xor_sync(0xffffffffu, mxx, o));
+    mxy = fmaxf(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
+    mxz = fmaxf(mxz, __shfl_xor_sync(0xffffffffu, mxz, o));
+  }
+  if (lane == 0) {
+    bb_c[w] = make_float4(0.5f * (mnx + mxx) + ox, 0.5f * (mny + mxy) + oy,
+                          0.5f * (mnz + mxz) + oz, 0.f);
+    bb_h[w] = make_float4(0.5f * (mxx - mnx), 0.5f * (mxy - mny), 0.5f * (mxz - mnz), 0.f);
+  }
 }
 
 // a new box for the built list: slot_off = k L - origin becomes k L' - origin
@@ -307,38 +337,6 @@ __global__ void refresh_kernel(const double4 *__restrict__ coords, const int *__
     out = make_float4((float)(c.x + o.x), (float)(c.y + o.y), (float)(c.z + o.z), (float)c.w);
   }
   xyzq_s[s] = out;
-}
-
-// (5) cluster bounding boxes, one warp per cluster
-__global__ void bbox_kernel(const float4 *__restrict__ xyzq_s, const int *__restrict__ perm,
-                            const float4 *__restrict__ cl_origin,
-                            float4 *__restrict__ bb_c, float4 *__restrict__ bb_h,
-                            const int *__restrict__ counts) {
-  int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  int lane = threadIdx.x & 31;
-  if (w >= counts[0] / kTile) return;
-  int s = w * kTile + lane;
-  float4 p = xyzq_s[s];
-  bool valid = perm[s] >= 0;
-  float mnx = valid ? p.x : INFINITY, mny = valid ? p.y : INFINITY,
-        mnz = valid ? p.z : INFINITY;
-  float mxx = valid ? p.x : -INFINITY, mxy = valid ? p.y : -INFINITY,
-        mxz = valid ? p.z : -INFINITY;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    mnx = fminf(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
-    mny = fminf(mny, __shfl_xor_sync(0xffffffffu, mny, o));
-    mnz = fminf(mnz, __shfl_xor_sync(0xffffffffu, mnz, o));
-    mxx = fmaxf(mxx, __shfl_xor_sync(0xffffffffu, mxx, o));
-    mxy = fmaxf(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
-    mxz = fmaxf(mxz, __shfl_xor_sync(0xffffffffu, mxz, o));
-  }
-  if (lane == 0) {
-    const float4 o = cl_origin[w];
-    bb_c[w] = make_float4(0.5f * (mnx + mxx) + o.x, 0.5f * (mny + mxy) + o.y,
-                          0.5f * (mnz + mxz) + o.z, 0.f);
-    bb_h[w] = make_float4(0.5f * (mxx - mnx), 0.5f * (mxy - mny), 0.5f * (mxz - mnz), 0.f);
-  }
 }
 
 // (6) tile search.  `split` warps per i-cluster, each with its share of the
@@ -748,12 +746,10 @@ void NeighborList::build(const float4 *d_xyzq, cudaStream_t s) {
                                             slot_shift, type_s, m_cl_col, m_col_sys, cl_sys,
                                             counts, m_d.sort_cap, d_xyzq);
   APO_LAUNCH_CHECK();
-  origin_kernel<<<(ncl * 32 + 255) / 256, 256, 0, s>>>(d_xyzq, perm, slot_shift, m_sys, cl_sys,
-                                                        cl_origin, slot_off, counts);
-  APO_LAUNCH_CHECK();
-  refresh(s);
-  bbox_kernel<<<(ncl * 32 + 255) / 256, 256, 0, s>>>(xyzq_s, perm, cl_origin, m_bb_c, m_bb_h,
-                                                      counts);
+  if (!m_coords) throw std::runtime_error("NeighborList: no state coordinates attached");
+  cluster_kernel<<<(ncl * 32 + 255) / 256, 256, 0, s>>>(d_xyzq, perm, slot_shift, m_sys, cl_sys,
+                                                         cl_origin, slot_off, m_coords, xyzq_s,
+                                                         m_bb_c, m_bb_h, counts);
   APO_LAUNCH_CHECK();
   const int split = m_d.split, tile_blocks = (int)(((long long)ncl * split * 32 + 127) / 128);
   tiles_kernel<false><<<tile_blocks, 128, 0, s>>>(
