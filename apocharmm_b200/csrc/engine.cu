@@ -1,7 +1,6 @@
 // ForceManager / CharmmContext; see engine.h.
 #include "engine.h"
 
-#include <climits>
 #include <type_traits>
 
 #include <algorithm>
@@ -144,10 +143,14 @@ __global__ void image_centering_kernel(double4 *__restrict__ c, float4 *__restri
   }
 }
 
+// first atom with a non-finite coordinate, or kNoBadAtom: above every atom
+// index, and made by a byte fill
+constexpr int kNoBadAtom = 0x7f7f7f7f;
+
 __global__ void coords_to_xyzq_kernel(const double4 *__restrict__ c, float4 *__restrict__ xq,
-                                      int n) {
+                                      int n, const int *__restrict__ bad) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
+  if (i < n && !(bad && *bad != kNoBadAtom)) {
     const double4 v = c[i];
     xq[i] = make_float4((float)v.x, (float)v.y, (float)v.z, (float)v.w);
   }
@@ -174,8 +177,9 @@ int order_components(std::vector<int2> &groups, int small) {
   return nbig;
 }
 
-void launch_coords_to_xyzq(const double4 *coords, float4 *xyzq, int n, cudaStream_t s) {
-  coords_to_xyzq_kernel<<<(n + 255) / 256, 256, 0, s>>>(coords, xyzq, n);
+void launch_coords_to_xyzq(const double4 *coords, float4 *xyzq, int n, cudaStream_t s,
+                           const int *bad) {
+  coords_to_xyzq_kernel<<<(n + 255) / 256, 256, 0, s>>>(coords, xyzq, n, bad);
   APO_LAUNCH_CHECK();
 }
 
@@ -364,6 +368,7 @@ void ForceManager::createStreams() {
     // whenever direct-space blocks retire
     int lo = 0, hi = 0;
     APO_CUDA(cudaDeviceGetStreamPriorityRange(&lo, &hi));
+    m_HostError.alloc();
     APO_CUDA(cudaStreamCreateWithPriority(&m_SNb, cudaStreamNonBlocking, lo));
     APO_CUDA(cudaStreamCreateWithPriority(&m_SPme, cudaStreamNonBlocking, hi));
     APO_CUDA(cudaStreamCreateWithPriority(&m_SBond, cudaStreamNonBlocking, hi));
@@ -535,8 +540,10 @@ void ForceManager::setPmeTensorCopies(bool on) {
 void ForceManager::calcForceChecked(const float4 *d_xyzq, bool calcEnergy, bool calcVirial,
                                     cudaStream_t s) {
   calcForce(d_xyzq, calcEnergy, calcVirial, s, true);
+  // the error word follows the kernels into pinned memory: one wait for both
+  APO_CUDA(cudaMemcpyAsync(m_HostError.p, m_Nbl.error, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
   APO_CUDA(cudaStreamSynchronize(s));
-  const unsigned e = readDeviceError(s);
+  const unsigned e = *m_HostError.p;
   if (e & kErrCopyTimeout)
     throw std::runtime_error("a tensor copy of the reciprocal-space grid did not complete");
   if (e & (kErrTileOverflow | kErrWorkOverflow)) {
@@ -977,7 +984,7 @@ __global__ void check_finite_kernel(const double *__restrict__ xyz, int n, int *
 __global__ void pack_xyz_kernel(const double *__restrict__ xyz, int n, double4 *__restrict__ out,
                                 const int *__restrict__ bad) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || (bad && *bad != INT_MAX)) return;
+  if (i >= n || (bad && *bad != kNoBadAtom)) return;
   double4 v = out[i];
   v.x = xyz[3 * i];
   v.y = xyz[3 * i + 1];
@@ -1011,8 +1018,9 @@ void CharmmContext::setCoordinatesXyz(const double *xyz, int first, int count, b
     throw std::invalid_argument("setCoordinates: atom range out of bounds");
   if (m_Stage.n != (size_t)3 * m_N) m_Stage.alloc((size_t)3 * m_N);
   if (m_BadAtom.n != 1) m_BadAtom.alloc(1);
-  const int ok = INT_MAX;
-  APO_CUDA(cudaMemcpyAsync(m_BadAtom.p, &ok, sizeof(int), cudaMemcpyHostToDevice, m_Stream));
+  m_HostBad.alloc();
+  static_assert(kNoBadAtom == 0x7f7f7f7f, "filled byte by byte");
+  APO_CUDA(cudaMemsetAsync(m_BadAtom.p, 0x7f, sizeof(int), m_Stream));
   APO_CUDA(cudaMemcpyAsync(m_Stage.p + 3 * (size_t)first, xyz, (size_t)3 * count * sizeof(double),
                            cudaMemcpyHostToDevice, m_Stream));
   const int b = (count + 255) / 256;
@@ -1024,20 +1032,22 @@ void CharmmContext::setCoordinatesXyz(const double *xyz, int first, int count, b
                                              m_Coords.p + first, m_BadAtom.p);
     APO_LAUNCH_CHECK();
   }
-  int bad = INT_MAX;
-  APO_CUDA(cudaMemcpyAsync(&bad, m_BadAtom.p, sizeof(int), cudaMemcpyDeviceToHost, m_Stream));
+  // like the state, the single-precision copies stay what they are if an atom
+  // was bad, so nothing waits for the verdict before the one wait for all
+  launch_coords_to_xyzq(m_Coords.p, m_Xyzq.p, m_N, m_Stream, m_BadAtom.p);
+  APO_CUDA(cudaMemcpyAsync(m_HostBad.p, m_BadAtom.p, sizeof(int), cudaMemcpyDeviceToHost, m_Stream));
   APO_CUDA(cudaStreamSynchronize(m_Stream));
-  if (bad != INT_MAX)
+  const int bad = *m_HostBad.p;
+  if (bad != kNoBadAtom)
     throw std::invalid_argument("setCoordinates: non-finite coordinate for atom " +
                                 std::to_string(first + bad));
-  launch_coords_to_xyzq(m_Coords.p, m_Xyzq.p, m_N, m_Stream);
   m_HasCoords = true;
   if (rebuild) {
     resetNeighborList(m_Stream);
+    APO_CUDA(cudaStreamSynchronize(m_Stream));
   } else {
     m_ListStale = true;
   }
-  APO_CUDA(cudaStreamSynchronize(m_Stream));
 }
 
 void CharmmContext::saveStateDevice(double4 *dst, int first, int count) {

@@ -65,6 +65,22 @@ struct DeviceArray {
   }
 };
 
+// One value in page-locked host memory, the target of small device-to-host
+// copies that are waited for together with the kernels before them.
+template <typename T>
+struct PinnedValue {
+  T *p = nullptr;
+  PinnedValue() = default;
+  void alloc() {
+    if (!p) APO_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&p), sizeof(T), cudaHostAllocDefault));
+  }
+  PinnedValue(const PinnedValue &) = delete;
+  PinnedValue &operator=(const PinnedValue &) = delete;
+  ~PinnedValue() {
+    if (p) cudaFreeHost(p);
+  }
+};
+
 // One system of a multi-system force manager (replicas, lambda windows, or
 // unrelated molecules advanced together): its files, box and nonbonded/PME
 // settings.  All systems of one manager share the spline order, the
@@ -278,6 +294,7 @@ class ForceManager {
   Topology m_Top;
 
   NeighborList m_Nbl;
+  PinnedValue<unsigned> m_HostError;  // the list's error word, copied behind an evaluation
   Pme m_Pme;
   int m_Stride = 0;
   DeviceArray<long long> m_Force, m_Energy;
@@ -372,7 +389,8 @@ class CharmmContext {
   DeviceArray<double4> m_Coords, m_VelMass;
   DeviceArray<float4> m_Xyzq;
   DeviceArray<double> m_Stage;    // 3N doubles: host transfers
-  DeviceArray<int> m_BadAtom;     // first non-finite coordinate, or INT_MAX
+  DeviceArray<int> m_BadAtom;     // first non-finite coordinate, or kNoBadAtom
+  PinnedValue<int> m_HostBad;     // its copy on the host
   DeviceArray<int2> m_Groups;
   int m_NumBigGroups = 0;  // leading components taken by a warp each
 };
@@ -385,6 +403,7 @@ void launch_image_centering(double4 *coords, float4 *xyzq, const int2 *groups, i
                             const int *sys_of_atom = nullptr, const double4 *boxes = nullptr);
 // stable reorder: components of more than `small` atoms first; returns their count
 int order_components(std::vector<int2> &groups, int small);
-void launch_coords_to_xyzq(const double4 *coords, float4 *xyzq, int n, cudaStream_t s);
+void launch_coords_to_xyzq(const double4 *coords, float4 *xyzq, int n, cudaStream_t s,
+                           const int *bad = nullptr);
 
 }  // namespace apo
