@@ -7,14 +7,16 @@
 // (:2381, body include/cuda_pme_gather.h), calc_self_energy (:2267).
 //
 // Pipeline (5 launches):
-//   spread      int32 fixed-point atomics into the real grid (deterministic)
+//   spread      int32 fixed-point sums into the real grid (deterministic): an
+//               atomic a point at order 4, patches of it at orders 6 and 8
 //   plane_fwd   one CTA per z-plane: R2C along x (two rows packed into one
 //               complex FFT), C2C along y; the plane lives in shared memory
 //   pencil      one CTA per (y-row, about 16 x-columns): FFT along z, multiply by
 //               the influence function (energy/virial reduced on the way),
 //               inverse FFT along z
 //   plane_inv   inverse of plane_fwd, writes the real potential grid
-//   gather      gradient from the potential, 8 threads per atom
+//   gather      gradient from the potential: a warp per atom at order 4, from a
+//               patch of the grid in shared memory at orders 6 and 8
 // The FFTs are in-place mixed-radix (2..8) shared-memory transforms.  A
 // decimation-in-frequency pass leaves its output in digit-reversed order and
 // a decimation-in-time pass takes digit-reversed input, so pairing them
