@@ -566,7 +566,7 @@ bool ForceManager::growNeighborList(const float4 *d_xyzq, cudaStream_t s) {
 }
 
 void ForceManager::calcForce(const float4 *d_xyzq, bool calcEnergy, bool calcVirial,
-                             cudaStream_t s, bool clear) {
+                             cudaStream_t s, bool clear, bool directEnergies) {
   if (!m_Initialized) throw std::runtime_error("ForceManager is not initialized");
   if (!m_ListBuilt || m_ListDirty) resetNeighborList(d_xyzq, s);
   else if (clear) m_Nbl.refresh(s);
@@ -631,7 +631,7 @@ void ForceManager::calcForce(const float4 *d_xyzq, bool calcEnergy, bool calcVir
       a.energy_stride = m_EStride;
       launch_nonbonded_multi(a, calcEnergy, m_Precise, m_SNb, calcVirial);
     } else {
-      launch_nonbonded(a, calcEnergy, m_Precise, m_SNb, calcVirial);
+      launch_nonbonded(a, calcEnergy && directEnergies, m_Precise, m_SNb, calcVirial);
     }
     if (t1) {
       if (timer_capture) APO_CUDA(cudaEventRecordWithFlags(t1, m_SNb, cudaEventRecordExternal));

@@ -85,7 +85,9 @@ class CudaIntegrator : public std::enable_shared_from_this<CudaIntegrator> {
   virtual void stepKernels(cudaStream_t s) = 0;  // the integration after forces
   void segment(int nsteps, cudaStream_t s);      // rebuild + nsteps steps
   void launchSegment(int nsteps, cudaStream_t s);  // as a captured graph (cached) or eagerly
-  virtual void forcesForStep(cudaStream_t s);
+  // forces of a step; `last`: the segment's last step, whose energies can be
+  // read afterwards
+  virtual void forcesForStep(cudaStream_t s, bool last);
   virtual void beforeReport() {}  // host state the subscribers read, after a synchronisation
   double m_Dt;  // AKMA
   int m_ListFreq = 20, m_ComFreq = 1000;
@@ -212,7 +214,7 @@ class CudaLangevinPistonIntegrator : public CudaIntegrator {
  protected:
   void initialize() override;
   void stepKernels(cudaStream_t s) override;
-  void forcesForStep(cudaStream_t s) override;  // with the virial
+  void forcesForStep(cudaStream_t s, bool last) override;  // with the virial
   void beforeReport() override;
   void adoptBox();  // the device's box into the force manager's host copies
   Crystal m_Crystal = Crystal::None;

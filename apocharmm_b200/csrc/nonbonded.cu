@@ -108,7 +108,6 @@ __device__ __forceinline__ void nb_body(const NbArgs &a) {
   const int nwork = a.counts[2];
   const int stride = a.stride;
   double e_elec = 0.0, e_vdw = 0.0;
-  double dv[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   // one system: per-lane fixed-point sums of every work item's energies and
   // virial (integer sums: the total does not depend on which warp took
   // which item)
@@ -394,10 +393,6 @@ __device__ __forceinline__ void nb_body(const NbArgs &a) {
         for (int k = 0; k < 6; ++k) vw[k] = -(f2lo(vw2[k]) + f2hi(vw2[k]));
       }
     }
-    if (VIRIAL) {
-#pragma unroll
-      for (int k = 0; k < 6; ++k) dv[k] += (double)vw[k];
-    }
     if (MULTI && ENERGY) {  // energies (and virial) belong to this work item's system
       long long *es = a.energy + (size_t)wk.w * a.energy_stride;
       warp_flush(e_elec, es + kEElec, lane);
@@ -408,14 +403,13 @@ __device__ __forceinline__ void nb_body(const NbArgs &a) {
         constexpr int kSlotM[6][2] = {{0, 0}, {1, 3}, {2, 6}, {4, 4}, {5, 7}, {8, 8}};
 #pragma unroll
         for (int k = 0; k < 6; ++k) {
-          long long iw = __double2ll_rn(dv[k] * kEnergyScale);
+          long long iw = __double2ll_rn((double)vw[k] * kEnergyScale);
 #pragma unroll
           for (int o = 16; o > 0; o >>= 1) iw += __shfl_xor_sync(0xffffffffu, iw, o);
           if (lane == 0 && iw) {
             add_fixed(es + kNumEnergyTerms + kSlotM[k][0], iw);
             if (kSlotM[k][1] != kSlotM[k][0]) add_fixed(es + kNumEnergyTerms + kSlotM[k][1], iw);
           }
-          dv[k] = 0.0;
         }
       }
     }
@@ -424,13 +418,10 @@ __device__ __forceinline__ void nb_body(const NbArgs &a) {
       ie_vdw += __double2ll_rn(e_vdw * kEnergyScale);
       e_elec = 0.0;
       e_vdw = 0.0;
-      if (VIRIAL) {
+    }
+    if (VIRIAL && !MULTI) {
 #pragma unroll
-        for (int k = 0; k < 6; ++k) {
-          ivir[k] += __double2ll_rn(dv[k] * kEnergyScale);
-          dv[k] = 0.0;
-        }
-      }
+      for (int k = 0; k < 6; ++k) ivir[k] += __double2ll_rn((double)vw[k] * kEnergyScale);
     }
     if (ivalid) {
       if (PER_PAIR) {
@@ -477,8 +468,8 @@ template <bool ENERGY, bool PER_PAIR, bool VIRIAL, bool MULTI>
 __global__ void __launch_bounds__(kThreads) nb_kernel(NbArgs a) {
   nb_body<ENERGY, PER_PAIR, VIRIAL, MULTI>(a);
 }
-// with energies the packed form is held to 128 registers, four blocks an SM: it
-// took 167 with the virial, three blocks (40 piston steps of 24,000 atoms 8.86
+// with energies or the virial the packed form is held to 128 registers, four
+// blocks an SM: it took 167 with both, three blocks (40 piston steps of 24,000 atoms 8.86
 // -> 8.70 ms, an evaluation with virial 603 -> 577 us).  Without energies the
 // compiler's own 122 (four blocks) stand.
 template <bool ENERGY, bool PER_PAIR, bool VIRIAL, bool MULTI>
@@ -854,14 +845,16 @@ void dispatch_q(const NbArgs &a, bool energy, bool per_pair, bool virial, cudaSt
 // reciprocal-space kernels, which cannot fill the GPU on their own at these
 // sizes, run beside it instead of after it (40 steps of 24,000 atoms 5.60 ->
 // 5.05 ms, of 42,000 6.37 -> 5.95, 20 steps of 53,000 5.36 -> 5.12, of 80,000
-// 7.47 -> 7.50, 40 of 107,000 15.35 -> 15.65).  Only without energies: that
-// kernel fills an SM's registers less evenly and loses (8.70 -> 9.08 ms).
+// 7.47 -> 7.50, 40 of 107,000 15.35 -> 15.65).  Only for the forces
+// alone: with energies (8.70 -> 9.08 ms) and with the virial (40 piston steps of
+// 24,000 atoms 7.86 -> 8.11, of 53,000 9.28 -> 9.26) the kernel is so much
+// longer than what runs beside it that it loses.
 constexpr int kSharedSmSlots = 65536;
 
 template <bool E, bool P, bool V = false, bool M = false>
 void launch_t(const NbArgs &a, cudaStream_t s) {
   void (*kernel)(NbArgs);
-  if constexpr (E && !P) kernel = nb_energy_kernel<E, P, V, M>;
+  if constexpr ((E || V) && !P) kernel = nb_energy_kernel<E, P, V, M>;
   else kernel = nb_kernel<E, P, V, M>;
   static int grid = 0, shared_grid = 0;
   size_t sm = M ? (size_t)kWarps * kMaxMultiTypes * kMaxMultiTypes * sizeof(float2)
@@ -875,7 +868,7 @@ void launch_t(const NbArgs &a, cudaStream_t s) {
     APO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, kThreads,
                                                            64 * 1024 > sm ? sm : 64 * 1024));
     grid = nsm * (per > 0 ? per : 1);
-    shared_grid = !E && per > 3 ? nsm * 3 : grid;
+    shared_grid = !E && !V && per > 3 ? nsm * 3 : grid;
   }
   const int resident = a.stride <= kSharedSmSlots ? shared_grid : grid;
   kernel<<<launch_grid(resident, a), kThreads, sm, s>>>(a);
@@ -892,9 +885,9 @@ void launch_nonbonded(const NbArgs &a, bool energy, bool per_pair, cudaStream_t 
   if (a.variant == kNbGroupedQueues) return dispatch_q<false>(a, energy, per_pair, virial, s);
   if (a.variant == kNbOctetLists) return launch_nonbonded_octets(a, energy, per_pair, virial, false, s);
   if (virial) {
-    if (!a.virial) throw std::invalid_argument("nonbonded: virial requested without a buffer");
     if (per_pair) launch_t<true, true, true>(a, s);
-    else launch_t<true, false, true>(a, s);
+    else if (energy) launch_t<true, false, true>(a, s);
+    else launch_t<false, false, true>(a, s);
     return;
   }
   if (per_pair) {

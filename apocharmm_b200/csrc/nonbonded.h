@@ -71,7 +71,8 @@ constexpr int kNbOctetLists = 2;
 // include/gpu_utils.h:281-312); otherwise FP32 sums per atom and tile are
 // rounded once (deterministic for a given tile list).
 // virial: also accumulate W = -sum over pairs of d (x) dU/dd into a.virial
-// (implies energy).
+// (with energies as well, except in the tile-batch form without per_pair of
+// one system, which leaves them out when `energy` is false).
 void launch_nonbonded(const NbArgs &a, bool energy, bool per_pair, cudaStream_t s,
                       bool virial = false);
 // every work item's system from its .w, with per-system LJ tables

@@ -171,3 +171,31 @@ def test_piston_step_equals_explicit_passes(tmp_path, passes):
     assert fm.getBoxDimensions() == pytest.approx([pos] * 3, abs=2e-8)
     assert np.abs(ctx.getCoordinates() - xx).max() < 2e-7
     assert np.abs(ctx.getVelocities() - (pred + p) / (2.0 * h)).max() < 2e-7 / h
+
+
+def test_piston_virial_without_energies(tmp_path):
+    """Within a segment the direct space leaves the energies out of the virial
+    kernel; with one-step segments every step takes the kernel with both.  The
+    lists differ (rebuilt every step or every 20), so single-precision sums
+    differ by their rounding: 1e-7 of the virial, 1e-8 A of an edge in a step."""
+    out = []
+    for freq in (1, 20):
+        s = water_box(600, 26.0, seed=8)
+        st = dict(kappa=0.34, nfft=(28, 28, 28), order=4, ctofnb=9.0, ctonnb=8.0, cutnb=11.0)
+        keep = api.system_context(s, str(tmp_path / f"f{freq}"), settings=st)
+        fm, ctx = keep[2], keep[3]
+        api.relax(ctx, api.water_indices(s), iterations=80)
+        ctx.setRandomSeedForVelocities(3)
+        ctx.assignVelocitiesAtTemperature(300.0)
+        it = api.CudaLangevinPistonIntegrator(0.001)
+        it.setCrystalType(it.CUBIC)
+        it.setNonbondedListUpdateFrequency(freq)
+        it.setCharmmContext(ctx)
+        it.propagate(10)
+        out.append((fm.getBoxDimensions(), ctx.getCoordinates(), ctx.getPotentialEnergy()))
+    assert abs(out[0][0][0] - s.box[0]) > 1e-6
+    assert out[0][0] == pytest.approx(out[1][0], abs=2e-7)
+    assert np.abs(out[0][1] - out[1][1]).max() < 1e-5
+    # the energies of the last step are there either way
+    assert out[0][2] == pytest.approx(out[1][2], rel=1e-5)
+    assert abs(out[1][2]) > 100.0
