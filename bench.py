@@ -629,8 +629,8 @@ def main():
                     help="z-pencil slabs by tiled tensor copies (1) or plain loads (0)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-e2e", action="store_true")
-    ap.add_argument("--tiles-per-work", type=int, default=8,
-                    help="j-tiles per direct-space work item")
+    ap.add_argument("--tiles-per-work", type=int, default=None,
+                    help="j-tiles per direct-space work item (default: the library's)")
     ap.add_argument("--items-per-warp", type=int, default=None,
                     help="direct-space work items per warp before it retires (0: persistent "
                          "grid; default: the library's)")
@@ -782,10 +782,9 @@ def main():
         if not args.no_cpu_baseline:
             cb = cpu_baseline(s)
         kps = integ.getKernelsPerStep()
-        if spec["integrator"] == "piston":  # the sorted coordinates refreshed every step
-            launches = args.steps * (12 + SEG * (8 + kps))
-        else:
-            launches = args.steps * (12 + SEG * (7 + kps))
+        # a segment: image centering and the list's eight launches, then per step
+        # direct space, five of PME, bonded and the integrator's own
+        launches = args.steps * (9 + SEG * (7 + kps))
         line = {
             "metric": "ns/day", "value": value, "unit": "ns/day", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": total_ms / args.steps,
