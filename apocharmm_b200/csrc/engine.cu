@@ -576,7 +576,8 @@ bool ForceManager::growNeighborList(const float4 *d_xyzq, cudaStream_t s) {
 }
 
 void ForceManager::calcForce(const float4 *d_xyzq, bool calcEnergy, bool calcVirial,
-                             cudaStream_t s, bool clear, bool directEnergies) {
+                             cudaStream_t s, bool clear, bool directEnergies,
+                             bool clearEnergies) {
   if (!m_Initialized) throw std::runtime_error("ForceManager is not initialized");
   if (!m_ListBuilt || m_ListDirty) resetNeighborList(d_xyzq, s);
   else if (clear) m_Nbl.refresh(s);
@@ -586,11 +587,13 @@ void ForceManager::calcForce(const float4 *d_xyzq, bool calcEnergy, bool calcVir
   // without energies no kernel of the evaluation touches the energy slots:
   // they are cleared beside it instead of before it
   if (!calcEnergy) APO_CUDA(cudaEventRecord(m_EvFork, s));
-  if (m_Multi)
-    APO_CUDA(cudaMemsetAsync(m_Energy.p, 0, m_Energy.n * sizeof(long long), s));
-  else
-    APO_CUDA(cudaMemsetAsync(m_Energy.p, 0,
-                             (kNumEnergyTerms + (calcVirial ? 9 : 0)) * sizeof(long long), s));
+  if (clearEnergies) {
+    if (m_Multi)
+      APO_CUDA(cudaMemsetAsync(m_Energy.p, 0, m_Energy.n * sizeof(long long), s));
+    else
+      APO_CUDA(cudaMemsetAsync(m_Energy.p, 0,
+                               (kNumEnergyTerms + (calcVirial ? 9 : 0)) * sizeof(long long), s));
+  }
   m_VirialValid = calcVirial;
   m_EvalMask = m_ComponentMask;
   if (calcEnergy) APO_CUDA(cudaEventRecord(m_EvFork, s));

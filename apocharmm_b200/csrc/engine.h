@@ -206,9 +206,10 @@ class ForceManager {
   void resetNeighborList(const float4 *d_xyzq, cudaStream_t s);
   // gradients into the slot-order fixed-point buffer (cleared first unless
   // clear == false); energies into the fixed-point energy slots
-  // (directEnergies = false: a virial whose direct-space energies nobody reads)
+  // (directEnergies = false: a virial whose direct-space energies nobody reads;
+  // clearEnergies = false: the energy and virial slots are known to be clear)
   void calcForce(const float4 *d_xyzq, bool calcEnergy, bool calcVirial, cudaStream_t s,
-                 bool clear = true, bool directEnergies = true);
+                 bool clear = true, bool directEnergies = true, bool clearEnergies = true);
   // FP64 state coordinates (x, y, z, q) in atom order, read by the bonded
   // terms; set by the CharmmContext that owns them
   void setStateCoordinates(const double4 *c) {

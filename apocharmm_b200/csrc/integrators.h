@@ -87,7 +87,7 @@ class CudaIntegrator : public std::enable_shared_from_this<CudaIntegrator> {
   void launchSegment(int nsteps, cudaStream_t s);  // as a captured graph (cached) or eagerly
   // forces of a step; `last`: the segment's last step, whose energies can be
   // read afterwards
-  virtual void forcesForStep(cudaStream_t s, bool last);
+  virtual void forcesForStep(cudaStream_t s, bool first, bool last);
   virtual void beforeReport() {}  // host state the subscribers read, after a synchronisation
   double m_Dt;  // AKMA
   int m_ListFreq = 20, m_ComFreq = 1000;
@@ -214,7 +214,7 @@ class CudaLangevinPistonIntegrator : public CudaIntegrator {
  protected:
   void initialize() override;
   void stepKernels(cudaStream_t s) override;
-  void forcesForStep(cudaStream_t s, bool last) override;  // with the virial
+  void forcesForStep(cudaStream_t s, bool first, bool last) override;  // with the virial
   void beforeReport() override;
   void adoptBox();  // the device's box into the force manager's host copies
   Crystal m_Crystal = Crystal::None;
@@ -226,6 +226,7 @@ class CudaLangevinPistonIntegrator : public CudaIntegrator {
   uint64_t m_Seed;
   unsigned long long m_RngPos = 0;
   bool m_RngDirty = true;
+  bool m_ClearEnergies = false;  // by the step being enqueued, for the next one
   std::unique_ptr<PistonState> m_P;
 };
 

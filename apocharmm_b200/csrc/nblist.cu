@@ -305,8 +305,10 @@ __global__ void rescale_dev_kernel(double4 *__restrict__ slot_off,
                                    const double *__restrict__ L0, const double *__restrict__ L1,
                                    const unsigned *__restrict__ err, const int *__restrict__ counts,
                                    const double4 *__restrict__ coords,
-                                   const int *__restrict__ perm, float4 *__restrict__ xyzq_s) {
+                                   const int *__restrict__ perm, float4 *__restrict__ xyzq_s,
+                                   long long *__restrict__ clear, int nclear) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (clear && s < nclear) clear[s] = 0;
   if (*err || s >= counts[0]) return;
   const int g = perm[s];
   const float4 o = cl_origin[s / kTile];
@@ -790,11 +792,13 @@ void NeighborList::set_box(int sys, double Lx, double Ly, double Lz) {
 }
 
 void NeighborList::rescale_box_device(const double *old_box, const double *new_box,
-                                      const unsigned *err, cudaStream_t s) {
+                                      const unsigned *err, cudaStream_t s, long long *clear,
+                                      int nclear) {
   if (m_sys_h.size() != 1) throw std::invalid_argument("NeighborList: one system only");
   if (!m_coords) throw std::runtime_error("NeighborList: no state coordinates attached");
   rescale_dev_kernel<<<(m_d.slot_cap + 255) / 256, 256, 0, s>>>(
-      slot_off, cl_origin, old_box, new_box, err, counts, m_coords, perm, xyzq_s);
+      slot_off, cl_origin, old_box, new_box, err, counts, m_coords, perm, xyzq_s,
+      clear, nclear);
   APO_LAUNCH_CHECK();
 }
 

@@ -105,7 +105,7 @@ class NeighborList {
   // in device memory (3 doubles each; nothing happens once `err` is set)
   // and the device dims are left alone
   void rescale_box_device(const double *old_box, const double *new_box, const unsigned *err,
-                          cudaStream_t s);
+                          cudaStream_t s, long long *clear, int nclear);
   // the host copy of a box the device dims already hold
   void set_box_host(int sys, double Lx, double Ly, double Lz);
   NbSysDims *device_dims() { return m_sys; }
