@@ -597,6 +597,21 @@ void ForceManager::calcForce(const float4 *d_xyzq, bool calcEnergy, bool calcVir
   m_VirialValid = calcVirial;
   m_EvalMask = m_ComponentMask;
   if (calcEnergy) APO_CUDA(cudaEventRecord(m_EvFork, s));
+  // the reciprocal space first: in a captured segment the first of the fork's
+  // kernels starts ahead of the others, and behind the direct-space grid the
+  // longer chain waited for it (40 steps of 24,000 atoms 5.90 -> 4.61 ms, at
+  // constant pressure 7.66 -> 6.78, of 12,500 2.49 -> 2.46, of 3,000 1.73 -> 1.65)
+  if (m_ComponentMask & 4) {
+    APO_CUDA(cudaStreamWaitEvent(m_SPme, m_EvFork, 0));
+    if (m_Multi)
+      m_PmeMulti.compute(m_Nbl.xyzq_s, m_Nbl.cl_origin, m_Nbl.cl_sys, m_Nbl.counts, m_Force.p,
+                         m_Stride, calcEnergy, calcVirial, m_Precise, m_SPme);
+    else
+      m_Pme.compute(m_Nbl.xyzq_s, m_Nbl.counts, m_Force.p, m_Stride, m_Energy.p, calcEnergy,
+                    m_Precise, m_SPme, virial, m_Nbl.cl_origin);
+    APO_CUDA(cudaEventRecord(m_EvPme, m_SPme));
+    APO_CUDA(cudaStreamWaitEvent(s, m_EvPme, 0));
+  }
   if (m_ComponentMask & 2) {
     APO_CUDA(cudaStreamWaitEvent(m_SNb, m_EvFork, 0));
     NbArgs a;
@@ -652,17 +667,6 @@ void ForceManager::calcForce(const float4 *d_xyzq, bool calcEnergy, bool calcVir
     }
     APO_CUDA(cudaEventRecord(m_EvNb, m_SNb));
     APO_CUDA(cudaStreamWaitEvent(s, m_EvNb, 0));
-  }
-  if (m_ComponentMask & 4) {
-    APO_CUDA(cudaStreamWaitEvent(m_SPme, m_EvFork, 0));
-    if (m_Multi)
-      m_PmeMulti.compute(m_Nbl.xyzq_s, m_Nbl.cl_origin, m_Nbl.cl_sys, m_Nbl.counts, m_Force.p,
-                         m_Stride, calcEnergy, calcVirial, m_Precise, m_SPme);
-    else
-      m_Pme.compute(m_Nbl.xyzq_s, m_Nbl.counts, m_Force.p, m_Stride, m_Energy.p, calcEnergy,
-                    m_Precise, m_SPme, virial, m_Nbl.cl_origin);
-    APO_CUDA(cudaEventRecord(m_EvPme, m_SPme));
-    APO_CUDA(cudaStreamWaitEvent(s, m_EvPme, 0));
   }
   // bonded terms proper; the 1-4 pairs and exclusion corrections go with
   // them or, under kComponent14WithDirect, with the direct space

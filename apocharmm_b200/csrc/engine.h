@@ -212,6 +212,7 @@ class ForceManager {
                  bool clear = true, bool directEnergies = true, bool clearEnergies = true);
   // FP64 state coordinates (x, y, z, q) in atom order, read by the bonded
   // terms; set by the CharmmContext that owns them
+  bool hasPlugins() const { return !m_Plugins.empty(); }
   void setStateCoordinates(const double4 *c) {
     m_StateCoords = c;
     m_Nbl.set_state_coordinates(c);

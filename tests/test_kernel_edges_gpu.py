@@ -199,3 +199,23 @@ def test_piston_virial_without_energies(tmp_path):
     # the energies of the last step are there either way
     assert out[0][2] == pytest.approx(out[1][2], rel=1e-5)
     assert abs(out[1][2]) > 100.0
+
+
+def test_steps_of_forces_alone_leave_the_energy_slots_clear(tmp_path):
+    """Only the first step of a segment clears the energy slots; with one-step
+    segments every step does."""
+    out = []
+    for freq in (1, 20):
+        s = water_box(600, 26.0, seed=8)
+        st = dict(kappa=0.34, nfft=(28, 28, 28), order=4, ctofnb=9.0, ctonnb=8.0, cutnb=11.0)
+        keep = api.system_context(s, str(tmp_path / f"f{freq}"), settings=st)
+        ctx = keep[3]
+        api.relax(ctx, api.water_indices(s), iterations=20)
+        ctx.assignVelocitiesAtTemperature(300.0)
+        it = api.CudaLangevinThermostatIntegrator(0.001)
+        it.setNonbondedListUpdateFrequency(freq)
+        it.setCharmmContext(ctx)
+        assert abs(ctx.calculatePotentialEnergy(True)) > 100.0
+        it.propagate(6)
+        out.append(ctx.getEnergyComponents())
+    assert out[0] == out[1]
