@@ -859,6 +859,7 @@ struct PistonArgs {
   double st;                     // surface tension x dyne/cm factor
   double ke_ref;
   int crystal, dof, use_nh, use_old, const_st, hol;
+  int keep_forces;               // leave the gradient slots for the caller
 };
 
 // piston move of one predictor-corrector pass (one thread)
@@ -1015,10 +1016,12 @@ __global__ void __launch_bounds__(kThreads) lp_half_kernel(Common c, PistonArgs 
   for (int j = 0; j < K; ++j) {
     o[j] = xyz(x[j]);
     du[j] = mk(0.0, 0.0, 0.0);
-    if (G.on[j]) {  // the slots are cleared for the next force evaluation
-      c.force[slot[j]] = 0;
-      c.force[c.stride + slot[j]] = 0;
-      c.force[2 * c.stride + slot[j]] = 0;
+    if (G.on[j]) {
+      if (!a.keep_forces) {  // the slots are cleared for the next force evaluation
+        c.force[slot[j]] = 0;
+        c.force[c.stride + slot[j]] = 0;
+        c.force[2 * c.stride + slot[j]] = 0;
+      }
       const d3 gr = mk((double)gi[j][0] * kInvForceScale, (double)gi[j][1] * kInvForceScale,
                        (double)gi[j][2] * kInvForceScale);
       du[j] = xyz(dp[j]) - (dt2 * vm[j].w) * gr;
@@ -2181,6 +2184,7 @@ void CudaLangevinPistonIntegrator::stepKernels(cudaStream_t s) {
   a.use_old = m_OldT ? 1 : 0;
   a.const_st = m_ConstST ? 1 : 0;
   a.hol = m_Ctx->isUsingHolonomicConstraints() ? 1 : 0;
+  a.keep_forces = m_LastStep ? 1 : 0;
   if (S.ngroups <= kFourLaneGroups) {
     lp_half_kernel<4><<<S.blocks_lanes, kThreads, 0, s>>>(S.c, a, m_MaxPC);
     lp_final_kernel<4><<<S.blocks_lanes, kThreads, 0, s>>>(S.c, a);
@@ -2193,11 +2197,13 @@ void CudaLangevinPistonIntegrator::stepKernels(cudaStream_t s) {
   fm->neighborList().rescale_box_device(
       reinterpret_cast<const double *>(ps + offsetof(PistonScalars, box_old)),
       reinterpret_cast<const double *>(ps + offsetof(PistonScalars, box)), S.c.err, s,
-      m_ClearEnergies ? fm->energyFixed() : nullptr, kNumEnergyTerms + 9);
+      m_LastStep ? nullptr : fm->energyFixed(), kNumEnergyTerms + 9);
 }
 
 void CudaLangevinPistonIntegrator::forcesForStep(cudaStream_t s, bool first, bool last) {
-  // forces and virial; the step kernels have cleared the gradient slots and
+  // forces and virial; the step kernels have cleared the gradient slots (but
+  // for the segment's last step, whose forces, energies and virial the caller
+  // can read; the next segment starts with a clear of its own) and
   // refreshed the sorted coordinates (the list build does at a segment's
   // start).  The direct-space energies (a third of that kernel's instructions)
   // go with the segment's last step only: the energy slots are cleared every
@@ -2208,7 +2214,7 @@ void CudaLangevinPistonIntegrator::forcesForStep(cudaStream_t s, bool first, boo
   // before it, those of the last stay for the caller (a clear of
   // their own stood before every step's forces: 40 steps of 24,000 atoms 7.81 ->
   // 7.58 ms, of 53,000 9.21 -> 9.03)
-  m_ClearEnergies = !last;
+  m_LastStep = last;
 }
 
 void CudaLangevinPistonIntegrator::adoptBox() {

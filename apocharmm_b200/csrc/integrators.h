@@ -226,7 +226,7 @@ class CudaLangevinPistonIntegrator : public CudaIntegrator {
   uint64_t m_Seed;
   unsigned long long m_RngPos = 0;
   bool m_RngDirty = true;
-  bool m_ClearEnergies = false;  // by the step being enqueued, for the next one
+  bool m_LastStep = false;  // of its segment: the step being enqueued
   std::unique_ptr<PistonState> m_P;
 };
 

@@ -201,6 +201,34 @@ def test_piston_virial_without_energies(tmp_path):
     assert abs(out[1][2]) > 100.0
 
 
+@pytest.mark.parametrize("steps", [1, 25])
+def test_piston_leaves_the_last_forces(tmp_path, steps):
+    """After a piston run the context holds the gradient of its last
+    evaluation, as it holds that evaluation's energies and virial."""
+    s = water_box(216, 19.0, seed=12)
+    st = dict(kappa=0.34, nfft=(20, 20, 20), order=4, ctofnb=8.0, ctonnb=7.0, cutnb=9.0)
+    keep = api.system_context(s, str(tmp_path), settings=st)
+    ctx = keep[3]
+    api.relax(ctx, api.water_indices(s), iterations=60)
+    ctx.assignVelocitiesAtTemperature(300.0)
+    it = api.CudaLangevinPistonIntegrator(0.001)
+    it.setCrystalType(it.CUBIC)
+    it.setCharmmContext(ctx)
+    if steps > 1:
+        it.propagate(steps - 1)
+    ctx.calculateForces(True, True, True)
+    g, e, w = ctx.getForces(), ctx.getEnergyComponents(), ctx.getVirial()
+    it.propagate(1)
+    # the same coordinates and box, a list built again: sums in another order
+    assert rel_rms(ctx.getForces(), g) < 1e-5
+    assert ctx.getEnergyComponents() == pytest.approx(e, rel=1e-5, abs=1e-3)
+    assert np.abs(ctx.getVirial() - w).max() < 1e-5 * np.abs(w).max()
+    # and within a longer segment: the last step's, not an earlier one's or none
+    it.propagate(3)
+    last = ctx.getForces()
+    assert np.abs(last).max() > 1.0 and rel_rms(last, g) > 1e-5
+
+
 def test_steps_of_forces_alone_leave_the_energy_slots_clear(tmp_path):
     """Only the first step of a segment clears the energy slots; with one-step
     segments every step does."""
