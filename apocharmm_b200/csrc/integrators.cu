@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "device_util.cuh"
+#include "step_record.h"
 
 namespace apo {
 
@@ -31,7 +32,7 @@ struct Scalars {
   long long step;
   long long window;
   unsigned counter;
-  unsigned pad;
+  StepRecord rec;            // of the step whose finishing launch is still to run
   double pc_a, pc_b;         // Nose-Hoover: displacement = pc_a delta + pc_b delta_prev
 };
 
@@ -311,6 +312,13 @@ __device__ void finish_temperature(const Common &c, double ke0, double ke1) {
   c.sc->window += 1;
 }
 
+// the end of a step's last kernel: what step_finish_kernel goes by (only
+// where the step was made: a kernel that found the error word set has returned)
+__device__ __forceinline__ void leave_step(const Common &c, const double (&ke)[2]) {
+  block_partials_n<2>(ke, c.partials);
+  if (blockIdx.x == 0 && threadIdx.x == 0) record_step(c.sc->rec);
+}
+
 // ------------------------------------------------------------ Langevin step
 // Position-Verlet "delta" Langevin of src/CudaLangevinThermostatIntegrator.cu:576-640:
 //   delta = alpha*delta_prev - dt^2/m/(1+g/2) * (grad + sqrt(2 g kT m)/dt * xi)
@@ -423,7 +431,7 @@ __global__ void __launch_bounds__(kThreads) langevin_kernel(Common c, double gam
                                  (float)(nk.z + so.z), (float)x.w);
   }
   const double ke[2] = {ke0, ke1};
-  block_partials_n<2>(ke, c.partials);  // summed by step_finish_kernel
+  leave_step(c, ke);
 }
 
 // ------------------------------------------------- groups on W lanes each
@@ -655,7 +663,7 @@ __global__ void __launch_bounds__(kThreads) nh_final_kernel(Common c) {
                                       (float)(n[j].z + so[j].z), (float)q[j]);
     }
   }
-  block_partials_n<2>(v, c.partials);  // summed by step_finish_kernel
+  leave_step(c, v);
 }
 
 // ---------------------------------------------------------------- leapfrog
@@ -676,7 +684,7 @@ __global__ void leapfrog_kernel(Common c, int natom) {
     ke1 = 0.5 * dot(nv, nv) / v.w;
   }
   const double ke[2] = {ke1, ke1};
-  block_partials_n<2>(ke, c.partials);  // summed by step_finish_kernel
+  leave_step(c, ke);
 }
 
 // ------------------------------------------------------- end of a step
@@ -690,7 +698,11 @@ enum FinishKind : int { kFinishLeapfrog, kFinishLangevin, kFinishNoseHoover };
 
 __global__ void __launch_bounds__(kThreads) step_finish_kernel(Common c, int blocks, int kind,
                                                                double ke_ref, int use_old) {
-  if (*c.err) return;
+  // not the error word: the next step's forces may be setting it (StepRecord)
+  __shared__ bool made;
+  if (threadIdx.x == 0) made = take_step(c.sc->rec);
+  __syncthreads();
+  if (!made) return;
   __shared__ double tot[2];
   sum_partials_n<2>(c.partials, blocks, tot);
   if (threadIdx.x == 0) {
