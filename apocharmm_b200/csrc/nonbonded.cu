@@ -25,6 +25,7 @@
 #include "device_util.cuh"
 #include "nblist.h"
 #include "nonbonded_pair.cuh"
+#include "resident_grid.h"
 
 namespace apo {
 
@@ -856,10 +857,9 @@ void launch_t(const NbArgs &a, cudaStream_t s) {
   void (*kernel)(NbArgs);
   if constexpr ((E || V) && !P) kernel = nb_energy_kernel<E, P, V, M>;
   else kernel = nb_kernel<E, P, V, M>;
-  static int grid = 0, shared_grid = 0;
   size_t sm = M ? (size_t)kWarps * kMaxMultiTypes * kMaxMultiTypes * sizeof(float2)
                 : (size_t)a.ntype * a.ntype * sizeof(float2);
-  if (!grid) {
+  const ResidentGrid &grid = resident_grid([&] {
     int dev, nsm, per = 0;
     APO_CUDA(cudaGetDevice(&dev));
     APO_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
@@ -867,10 +867,12 @@ void launch_t(const NbArgs &a, cudaStream_t s) {
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
     APO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, kThreads,
                                                            64 * 1024 > sm ? sm : 64 * 1024));
-    grid = nsm * (per > 0 ? per : 1);
-    shared_grid = !E && !V && per > 3 ? nsm * 3 : grid;
-  }
-  const int resident = a.stride <= kSharedSmSlots ? shared_grid : grid;
+    ResidentGrid g;
+    g.full = nsm * (per > 0 ? per : 1);
+    g.shared = !E && !V && per > 3 ? nsm * 3 : g.full;
+    return g;
+  });
+  const int resident = a.stride <= kSharedSmSlots ? grid.shared : grid.full;
   kernel<<<launch_grid(resident, a), kThreads, sm, s>>>(a);
   APO_LAUNCH_CHECK();
 }

@@ -1,8 +1,14 @@
 // Host-side rules of the engine, run without a device:
 //   host_rules step   the counters follow the steps that were made
+//   host_rules grid   threads that launch a kernel form first, together
+#include <atomic>
+#include <chrono>
 #include <cstdio>
 #include <cstring>
+#include <thread>
+#include <vector>
 
+#include "resident_grid.h"
 #include "step_record.h"
 
 namespace {
@@ -38,9 +44,36 @@ int step() {
   return 0;
 }
 
+int grid() {
+  std::atomic<int> asked{0}, ready{0}, wrong{0};
+  auto launch = [&] {
+    ++ready;
+    while (ready < 8) std::this_thread::yield();
+    const apo::ResidentGrid &g = apo::resident_grid([&asked] {
+      ++asked;
+      apo::ResidentGrid r;
+      std::this_thread::sleep_for(std::chrono::milliseconds(20));
+      r.full = 592;
+      std::this_thread::sleep_for(std::chrono::milliseconds(20));
+      r.shared = 444;
+      return r;
+    });
+    if (g.full != 592 || g.shared != 444) ++wrong;
+  };
+  std::vector<std::thread> t;
+  for (int k = 0; k < 8; ++k) t.emplace_back(launch);
+  for (auto &x : t) x.join();
+  if (asked != 1 || wrong != 0) {
+    std::printf("asked %d times, %d threads saw half an answer\n", asked.load(), wrong.load());
+    return 1;
+  }
+  return 0;
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
   if (argc == 2 && !std::strcmp(argv[1], "step")) return step();
+  if (argc == 2 && !std::strcmp(argv[1], "grid")) return grid();
   return 2;
 }

@@ -12,7 +12,7 @@ CXX = shutil.which("g++")
 
 
 @pytest.mark.skipif(CXX is None, reason="g++ not found")
-@pytest.mark.parametrize("rule", ["step"])
+@pytest.mark.parametrize("rule", ["step", "grid"])
 def test_host_rule(tmp_path, rule):
     exe = str(tmp_path / "host_rules")
     r = subprocess.run([CXX, "-std=c++17", "-O1", "-Wall", "-Werror", "-pthread", "-I",
