@@ -240,6 +240,8 @@ class Oracle:
         L = lib()
         xyz = np.ascontiguousarray(self.sys.pos if pos is None else pos, np.float64).reshape(-1)
         n = self.n
+        if not np.isfinite(xyz).all():  # the cell lists are indexed by them
+            raise ValueError("non-finite coordinates")
         grad_all = np.zeros(3 * n)
         vir = np.zeros(9)
         grad = np.zeros(3 * n) if virial else grad_all

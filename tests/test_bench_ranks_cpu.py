@@ -7,11 +7,14 @@ import subprocess
 import sys
 import types
 
+import numpy as np
 import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 sys.path.insert(0, ROOT)
 import bench  # noqa: E402
+import oracle  # noqa: E402
+from apocharmm_b200.systems import water_box  # noqa: E402
 
 CHILD = r"""
 import os, sys, datetime
@@ -98,3 +101,32 @@ def test_gpus_flag_must_match_world_size():
                        timeout=120)
     assert r.returncode == 2
     assert "WORLD_SIZE" in r.stderr
+
+
+def test_reference_arm_without_its_build_says_so(monkeypatch, capsys):
+    """The generated structure has close contacts that only the reference's
+    build relaxes: without that build the arm names the reason, gives no value
+    for the reference, and its host baseline does not fly apart."""
+    import json
+    s = water_box(400, 23.0, seed=3)
+    s.pos = s.pos + np.random.default_rng(1).normal(0.0, 0.25, s.pos.shape)
+    s.settings = dict(kappa=0.34, nfft=(24, 24, 24), order=4, ctofnb=9.0, ctonnb=7.5, cutnb=11.0)
+    monkeypatch.setattr(bench, "make_system", lambda name: s)
+    monkeypatch.setattr(bench.os.path, "exists",
+                        lambda p, real=os.path.exists: "ref_harness" not in str(p) and real(p))
+    for k in ("RANK", "WORLD_SIZE", "LOCAL_RANK"):
+        monkeypatch.delenv(k, raising=False)
+    args = types.SimpleNamespace(workload="water12k", gpus=1, steps=1, warmup=3)
+    assert bench.run_reference_arm(args) == 0
+    line = json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and "not present" in line["unavailable"]
+    assert "value" not in line and "e2e" not in line
+    assert line["cpu_baseline"]["value"] > 0.0
+
+
+def test_oracle_refuses_non_finite_coordinates():
+    s = water_box(27, 10.0, seed=1)
+    x = s.pos.copy()
+    x[5, 1] = np.nan
+    with pytest.raises(ValueError, match="non-finite"):
+        oracle.Oracle(s, 0.34, 4.5, 4.0, (12, 12, 12), 4).evaluate(pos=x)
