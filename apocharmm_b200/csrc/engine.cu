@@ -195,7 +195,7 @@ ForceManager::ForceManager(const std::vector<SystemSpec> &systems, int order, in
     : m_Multi(true), m_Specs(systems) {
   if (systems.empty()) throw std::invalid_argument("ForceManager: no systems");
   m_Order = order;
-  m_TilesPerWork = std::max(1, tilesPerWork);
+  m_TilesPerWork = tilesPerWork;
   m_Precise = precise;
   initializeMulti();
 }
@@ -339,7 +339,7 @@ void ForceManager::initialize() {
   m_Setup.upload(std::vector<NbSetup>{m_HostSetup});
 
   m_Nbl.setup(n, m_Box[0], m_Box[1], m_Box[2], (float)m_Cutoff,
-              m_Top.excl_ptr, m_Top.excl_idx, m_VdwTypeD.p, tilesPerWork(n));
+              m_Top.excl_ptr, m_Top.excl_idx, m_VdwTypeD.p, m_TilesPerWork);
   m_Pme.setup(m_Nfft[0], m_Nfft[1], m_Nfft[2], m_Order, m_Kappa, m_Box[0], m_Box[1], m_Box[2]);
   m_Pme.max_slots = m_Nbl.dims().slot_cap;
   m_Pme.set_error_word(m_Nbl.error);
@@ -359,16 +359,6 @@ void ForceManager::initialize() {
   m_ListBuilt = false;
   m_Initialized = true;
   for (auto &p : m_Plugins) p.second->initialize(m_Top.natom, m_Box);
-}
-
-// A work item's i-atoms are loaded, and its queue's last batch is padded, once
-// whatever its length, so long lists take longer items; short ones need the
-// items to fill the GPU evenly.  8 -> 16 tiles: 40 steps of 3,000 atoms 1.76 ->
-// 2.31 ms, of 24,000 4.96 -> 5.22, of 47,000 6.68 -> 6.61; 20 steps of 107,000
-// 8.08 -> 7.91, of 998,000 55.98 -> 53.76 (32 tiles: 7.97 and 53.28).
-int ForceManager::tilesPerWork(int natom) const {
-  if (m_TilesPerWork > 0) return m_TilesPerWork;
-  return natom >= 65536 ? 16 : 8;
 }
 
 void ForceManager::createStreams() {
@@ -504,7 +494,7 @@ void ForceManager::initializeMulti() {
   m_Setup.upload(setups);
   m_Boxes.upload(boxes);
 
-  m_Nbl.setup(lists, m_Top.excl_ptr, m_Top.excl_idx, m_VdwTypeD.p, tilesPerWork(m_Top.natom));
+  m_Nbl.setup(lists, m_Top.excl_ptr, m_Top.excl_idx, m_VdwTypeD.p, m_TilesPerWork);
   m_Stride = m_Nbl.dims().slot_cap;
   m_Force.alloc((size_t)3 * m_Stride);
   APO_CUDA(cudaMemset(m_Force.p, 0, (size_t)3 * m_Stride * sizeof(long long)));

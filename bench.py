@@ -632,8 +632,8 @@ def main():
                     help="z-pencil slabs by tiled tensor copies (1) or plain loads (0)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-e2e", action="store_true")
-    ap.add_argument("--tiles-per-work", type=int, default=None,
-                    help="j-tiles per direct-space work item (default: the library's)")
+    ap.add_argument("--tiles-per-work", type=int, default=8,
+                    help="j-tiles per direct-space work item (8: the library's default)")
     ap.add_argument("--items-per-warp", type=int, default=None,
                     help="direct-space work items per warp before it retires (0: persistent "
                          "grid; default: the library's)")

@@ -71,6 +71,22 @@ def test_direct_space_remainders(tmp_path, n, ron):
             assert np.abs(ctx.getVirial() - W).max() < 1e-6 * max(20.0, np.abs(W).max())
 
 
+def test_default_work_items_of_a_large_box(tmp_path):
+    """An i-atom's single-precision sum runs over a work item: its length does not
+    grow with the system unless the caller asks for it."""
+    n = 22000                                 # 66,000 atoms
+    s = water_box(n, (3 * n / 0.1003) ** (1.0 / 3.0), seed=4)
+    st = dict(kappa=0.34, nfft=(90, 90, 90), order=4, ctofnb=8.0, ctonnb=7.0, cutnb=9.0)
+    g = {}
+    for tiles in (None, 8, 16):
+        keep = api.system_context(s, str(tmp_path / str(tiles)), settings=st, tiles_per_work=tiles)
+        keep[2].setComponentMask(2)
+        keep[3].calculateForces(False, False, False)
+        g[tiles] = keep[3].getForces()
+    assert np.array_equal(g[None], g[8])
+    assert 0.0 < rel_rms(g[16], g[8]) < 1e-6
+
+
 def _flexible(tmp_path, dt, make):
     s = water_box(216, 19.0, seed=12)
     st = dict(kappa=0.34, nfft=(20, 20, 20), order=4, ctofnb=8.0, ctonnb=7.0, cutnb=9.0)
