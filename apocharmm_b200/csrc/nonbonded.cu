@@ -846,11 +846,16 @@ void dispatch_q(const NbArgs &a, bool energy, bool per_pair, bool virial, cudaSt
 // reciprocal-space kernels, which cannot fill the GPU on their own at these
 // sizes, run beside it instead of after it (40 steps of 24,000 atoms 5.60 ->
 // 5.05 ms, of 42,000 6.37 -> 5.95, 20 steps of 53,000 5.36 -> 5.12, of 80,000
-// 7.47 -> 7.50, 40 of 107,000 15.35 -> 15.65).  Only for the forces
+// 7.47 -> 7.50, 40 of 107,000 15.35 -> 15.65; batches of 3 systems of 3,000
+// atoms 1.35 -> 1.28 ms, of 12 3.18 -> 3.13, of 8 at order 6 3.47 -> 3.27).
+// The precise form's kernel is longer and pays only at the smallest sizes (20
+// Langevin steps at order 4 of 3,000 atoms 1.44 -> 1.30 ms, of 6,000 1.52 ->
+// 1.43, of 9,000 1.69 -> 1.70, of 12,000 1.93 -> 1.99, of 24,000 2.98 -> 3.17;
+// a batch of 12 systems of 3,000 4.18 -> 4.44).  Only for the forces
 // alone: with energies (8.70 -> 9.08 ms) and with the virial (40 piston steps of
 // 24,000 atoms 7.86 -> 8.11, of 53,000 9.28 -> 9.26) the kernel is so much
 // longer than what runs beside it that it loses.
-constexpr int kSharedSmSlots = 65536;
+constexpr int kSharedSmSlots = 65536, kSharedSmSlotsPrecise = 10240;
 
 template <bool E, bool P, bool V = false, bool M = false>
 void launch_t(const NbArgs &a, cudaStream_t s) {
@@ -872,7 +877,7 @@ void launch_t(const NbArgs &a, cudaStream_t s) {
     g.shared = !E && !V && per > 3 ? nsm * 3 : g.full;
     return g;
   });
-  const int resident = a.stride <= kSharedSmSlots ? grid.shared : grid.full;
+  const int resident = a.stride <= (P ? kSharedSmSlotsPrecise : kSharedSmSlots) ? grid.shared : grid.full;
   kernel<<<launch_grid(resident, a), kThreads, sm, s>>>(a);
   APO_LAUNCH_CHECK();
 }
