@@ -210,7 +210,6 @@ class ForceManager {
   // clearEnergies = false: the energy and virial slots are known to be clear)
   void calcForce(const float4 *d_xyzq, bool calcEnergy, bool calcVirial, cudaStream_t s,
                  bool clear = true, bool directEnergies = true, bool clearEnergies = true);
-  bool hasPlugins() const { return !m_Plugins.empty(); }
   // FP64 state coordinates (x, y, z, q) in atom order, read by the bonded
   // terms; set by the CharmmContext that owns them
   void setStateCoordinates(const double4 *c) {

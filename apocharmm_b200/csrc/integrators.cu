@@ -1482,11 +1482,11 @@ void CudaIntegrator::buildGroups() {
 
 void CudaIntegrator::forcesForStep(cudaStream_t s, bool first, bool) {
   // only the first step of a segment clears the energy slots: evaluations of
-  // forces alone leave them so, except for a plug-in's.  A clear in every step, even
-  // beside the forces, held up the graph and made it one branch wider (a first
-  // pass of 3,000 atoms 3.64 -> 2.57 ms, a steady one 1.75 -> 1.65)
-  auto fm = m_Ctx->getForceManager();
-  fm->calcForce(m_Ctx->xyzq(), false, false, s, /*clear=*/false, true, first || fm->hasPlugins());
+  // forces alone leave them so (a plug-in's energy has a slot elsewhere).  A
+  // clear in every step, even beside the forces, held up the graph and made it
+  // one branch wider (a first pass of 3,000 atoms 3.64 -> 2.57 ms, a steady one
+  // 1.75 -> 1.65, with a restraint subscribed 2.15 -> 1.74)
+  m_Ctx->getForceManager()->calcForce(m_Ctx->xyzq(), false, false, s, /*clear=*/false, true, first);
 }
 
 void CudaIntegrator::segment(int nsteps, cudaStream_t s) {

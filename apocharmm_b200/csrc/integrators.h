@@ -85,8 +85,8 @@ class CudaIntegrator : public std::enable_shared_from_this<CudaIntegrator> {
   virtual void stepKernels(cudaStream_t s) = 0;  // the integration after forces
   void segment(int nsteps, cudaStream_t s);      // rebuild + nsteps steps
   void launchSegment(int nsteps, cudaStream_t s);  // as a captured graph (cached) or eagerly
-  // forces of a step; `last`: the segment's last step, whose energies can be
-  // read afterwards
+  // forces of a step; `first`: the segment's first step, which clears the
+  // energy slots; `last`: its last step, whose energies can be read afterwards
   virtual void forcesForStep(cudaStream_t s, bool first, bool last);
   virtual void beforeReport() {}  // host state the subscribers read, after a synchronisation
   double m_Dt;  // AKMA

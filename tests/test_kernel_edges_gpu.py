@@ -245,9 +245,10 @@ def test_piston_leaves_the_last_forces(tmp_path, steps):
     assert np.abs(last).max() > 1.0 and rel_rms(last, g) > 1e-5
 
 
-def test_steps_of_forces_alone_leave_the_energy_slots_clear(tmp_path):
-    """Only the first step of a segment clears the energy slots; with one-step
-    segments every step does."""
+@pytest.mark.parametrize("restraint", [False, True])
+def test_steps_of_forces_alone_leave_the_energy_slots_clear(tmp_path, restraint):
+    """Only the first step of a segment clears the energy slots, plug-in forces or
+    not; with one-step segments every step does."""
     out = []
     for freq in (1, 20):
         s = water_box(600, 26.0, seed=8)
@@ -256,10 +257,22 @@ def test_steps_of_forces_alone_leave_the_energy_slots_clear(tmp_path):
         ctx = keep[3]
         api.relax(ctx, api.water_indices(s), iterations=20)
         ctx.assignVelocitiesAtTemperature(300.0)
+        if restraint:
+            hold = api.HarmonicRestraintForce(s.n_atoms)
+            hold.setReferenceCoordinates(ctx.getCoordinates() + 0.1)
+            hold.setSelection(np.arange(3))
+            hold.setForceConstant(1.0)
+            keep[2].subscribe(hold, "hold")
         it = api.CudaLangevinThermostatIntegrator(0.001)
         it.setNonbondedListUpdateFrequency(freq)
         it.setCharmmContext(ctx)
         assert abs(ctx.calculatePotentialEnergy(True)) > 100.0
+        held = ctx.getEnergyComponent("hold") if restraint else 0.0
         it.propagate(6)
         out.append(ctx.getEnergyComponents())
+        # all but the self energy, which is no slot; the plug-in's own slot keeps
+        # its last evaluated energy
+        assert all(v == 0.0 for k, v in out[-1].items() if k != "ewse")
+        if restraint:
+            assert ctx.getEnergyComponent("hold") == held > 0.0
     assert out[0] == out[1]
