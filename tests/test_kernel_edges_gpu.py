@@ -19,7 +19,9 @@ ATMOSP = 1.4584007e-05
 @pytest.mark.parametrize("nfft,order", [((16, 18, 20), 4), ((18, 16, 24), 6), ((20, 28, 30), 4),
                                         ((42, 40, 50), 6), ((50, 56, 36), 8), ((70, 40, 98), 4),
                                         ((64, 64, 64), 6), ((128, 100, 60), 4),
-                                        ((90, 216, 32), 6), ((216, 180, 48), 4)])
+                                        ((90, 216, 32), 6), ((216, 180, 48), 4),
+                                        # no room for the twiddles beside the plane
+                                        ((256, 224, 16), 4), ((224, 252, 18), 6)])
 def test_reciprocal_space_on_many_grids(tmp_path, nfft, order):
     s = water_box(300, 21.0, seed=9)
     st = dict(kappa=0.34, nfft=nfft, order=order, ctofnb=8.0, ctonnb=7.0, cutnb=9.0)
@@ -87,9 +89,27 @@ def test_default_work_items_of_a_large_box(tmp_path):
     assert 0.0 < rel_rms(g[16], g[8]) < 1e-6
 
 
-def _flexible(tmp_path, dt, make):
-    s = water_box(216, 19.0, seed=12)
-    st = dict(kappa=0.34, nfft=(20, 20, 20), order=4, ctofnb=8.0, ctonnb=7.0, cutnb=9.0)
+SMALL = 216     # waters: integrator kernels with four lanes a group
+# more than 65,536 groups, of a water or of four free atoms: one lane a group,
+# the direct-space grid that fills every SM
+LARGE = 87500
+
+
+def _water(n):
+    """n waters and settings; thermostat and piston masses under which a step
+    moves them alike at every n."""
+    if n == SMALL:
+        return (water_box(n, 19.0, seed=12),
+                dict(kappa=0.34, nfft=(20, 20, 20), order=4, ctofnb=8.0, ctonnb=7.0, cutnb=9.0),
+                2.0, 50.0)
+    L = (3 * n / 0.1003) ** (1.0 / 3.0)
+    return (water_box(n, L, seed=12),
+            dict(kappa=0.34, nfft=(144, 144, 144), order=4, ctofnb=8.0, ctonnb=7.0, cutnb=9.0),
+            2.0 * n / SMALL, 50.0 * (L / 19.0) ** 2)
+
+
+def _flexible(tmp_path, dt, make, n=SMALL):
+    s, st, nh_mass, _ = _water(n)
     keep = api.system_context(s, str(tmp_path), settings=st)
     fm, ctx = keep[2], keep[3]
     api.relax(ctx, None, iterations=60)
@@ -102,16 +122,18 @@ def _flexible(tmp_path, dt, make):
     g, W = ctx.getForces(), ctx.getVirial()
     it = make(dt)
     it.setReferenceTemperature(300.0)
-    it.setNoseHooverPistonMass(2.0)   # light: the passes differ by more than rounding
+    it.setNoseHooverPistonMass(nh_mass)   # light: the passes differ by more than rounding
     it.setCharmmContext(ctx)
     it.propagate(1)
     return s, keep, it, x, v, g, W, dt / TIMFAC
 
 
-def test_nose_hoover_step_equals_explicit_passes(tmp_path):
+@pytest.mark.parametrize("n", [SMALL, LARGE])
+def test_nose_hoover_step_equals_explicit_passes(tmp_path, n):
     """One unconstrained step: the scalar predictor-corrector passes against
     three explicit passes over the atoms."""
-    s, keep, it, x, v, g, W, h = _flexible(tmp_path, 0.001, api.CudaNoseHooverIntegrator)
+    s, keep, it, x, v, g, W, h = _flexible(tmp_path, 0.001, api.CudaNoseHooverIntegrator, n)
+    nh_mass = _water(n)[2]
     m = s.mass[:, None]
     p = h * v + 0.5 * h * h * g / m          # delta_prev from velocities and first forces,
     p -= (m * p).sum(0) / m.sum()            # without the drift, removed at step 0
@@ -123,7 +145,7 @@ def test_nose_hoover_step_equals_explicit_passes(tmp_path):
 
     ke, xi, pred = three(v), 0.0, d
     for k in range(3):
-        f = 2.0 * h * (ke - ke_ref) / 2.0
+        f = 2.0 * h * (ke - ke_ref) / nh_mass
         xi = 0.0 + 0.5 * (f + (f if k == 0 else f0))
         f0 = f if k == 0 else f0             # the previous force starts as the first one
         u = (p + pred) / (2.0 * h)
@@ -137,18 +159,20 @@ def test_nose_hoover_step_equals_explicit_passes(tmp_path):
     assert np.abs(keep[3].getVelocities() - (pred + p) / (2.0 * h)).max() < 2e-7 / h
 
 
-@pytest.mark.parametrize("passes", [1, 2, 3, 4])
-def test_piston_step_equals_explicit_passes(tmp_path, passes):
+@pytest.mark.parametrize("passes,n", [(1, SMALL), (2, SMALL), (3, SMALL), (4, SMALL), (3, LARGE)])
+def test_piston_step_equals_explicit_passes(tmp_path, passes, n):
     """One unconstrained cubic step without piston friction: box, coordinates
     and velocities against explicit passes over the atoms."""
+    nh_mass, lp_mass = _water(n)[2:]
+
     def make(dt):
         it = api.CudaLangevinPistonIntegrator(dt)
         it.setCrystalType(it.CUBIC)
-        it.setLangevinPistonMass([50.0])
+        it.setLangevinPistonMass([lp_mass])
         it.setMaxPredictorCorrectorIterations(passes)
         return it
 
-    s, keep, it, x, v, g, W, h = _flexible(tmp_path, 0.001, make)
+    s, keep, it, x, v, g, W, h = _flexible(tmp_path, 0.001, make, n)
     fm, ctx = keep[2], keep[3]
     m = s.mass[:, None]
     p = h * v + 0.5 * h * h * g / m
@@ -169,11 +193,11 @@ def test_piston_step_equals_explicit_passes(tmp_path, passes):
     pred, r = d, x
     xx = r + d
     for k in range(passes):
-        delta = (1.0 / 50.0) * (np.trace(dp) / L) * V * h * h * ATMOSP
+        delta = (1.0 / lp_mass) * (np.trace(dp) / L) * V * h * h * ATMOSP
         onvel = 0.5 * delta / h
         pos = L + delta
         on, half = h * onvel / L, delta / (pos - 0.5 * delta)
-        f = 2.0 * h * (ke - ke_ref) / 2.0
+        f = 2.0 * h * (ke - ke_ref) / nh_mass
         f0 = f if k == 0 else f0
         xi = 0.5 * (f + f0)
         u = (p + pred) / (2.0 * h)
@@ -187,6 +211,53 @@ def test_piston_step_equals_explicit_passes(tmp_path, passes):
     assert fm.getBoxDimensions() == pytest.approx([pos] * 3, abs=2e-8)
     assert np.abs(ctx.getCoordinates() - xx).max() < 2e-7
     assert np.abs(ctx.getVelocities() - (pred + p) / (2.0 * h)).max() < 2e-7 / h
+
+
+@pytest.mark.parametrize("kind", ["nose_hoover", "piston"])
+def test_one_lane_a_group_holds_the_constraints(tmp_path, kind):
+    s, st, _, _ = _water(LARGE)
+    keep = api.system_context(s, str(tmp_path), settings=st)
+    ctx = keep[3]
+    w = api.water_indices(s)
+    api.relax(ctx, w, iterations=60)
+    ctx.assignVelocitiesAtTemperature(300.0)
+    if kind == "piston":
+        it = api.CudaLangevinPistonIntegrator(0.002)
+        it.setCrystalType(it.CUBIC)
+    else:
+        it = api.CudaNoseHooverIntegrator(0.002)
+    it.setReferenceTemperature(300.0)
+    it.setCharmmContext(ctx)
+    it.propagate(25)
+    x, v = ctx.getCoordinates().reshape(-1, 3, 3), ctx.getVelocities()
+    d = np.linalg.norm(x[:, [0, 0, 1]] - x[:, [1, 2, 2]], axis=2)
+    # SETTLE works in FP64 on coordinates of up to 70 A: 1e-14 of them, squared
+    # lengths of 1 A^2 to 1e-12
+    assert np.abs(d - d[0]).max() < 1e-9
+    drift = (s.mass[:, None] * v).sum(0) / np.abs(s.mass[:, None] * v).sum(0)
+    # each force is rounded to 2^-40 kcal/mol/A, pairs are equal and opposite;
+    # the reciprocal space leaves a net force of about 1e-5 of an atom's
+    assert np.abs(drift).max() < 1e-4
+    assert 200.0 < it.getInstantaneousTemperature() < 2000.0
+
+
+def test_direct_space_of_a_large_box(tmp_path):
+    """Work items of 8 and 16 tiles on a grid that fills every SM, against 64
+    bits."""
+    s, st, _, _ = _water(LARGE)
+    for tiles in (8, 16):
+        keep = api.system_context(s, str(tmp_path / str(tiles)), settings=st, tiles_per_work=tiles)
+        fm, ctx = keep[2], keep[3]
+        if tiles == 8:
+            s.pos = api.relax(ctx, api.water_indices(s), iterations=40)
+            E, G, W = oracle_for(s, st).evaluate(parts=("direct",), virial=True)
+        fm.setComponentMask(2)
+        for energy, virial in ((False, False), (True, True)):
+            ctx.calculateForces(True, energy, virial)
+            # 6.3e-7 to 7.7e-7 measured in larger and longer-ranged boxes
+            assert rel_rms(ctx.getForces(), G) < 3e-6
+        assert ctx.getPotentialEnergy() == pytest.approx(E["epot"], rel=1e-6)
+        assert np.abs(ctx.getVirial() - W).max() < 1e-6 * np.abs(W).max()
 
 
 def test_piston_virial_without_energies(tmp_path):
