@@ -252,8 +252,11 @@ __device__ __forceinline__ float2 twiddle(const float2 *tw, int idx) {
 // their shared-memory accesses are lstride apart, free of bank conflicts for
 // columns (lstride 1; with consecutive threads along a line the z pencils,
 // estride 16, hit one bank with half a warp: 14.5 us a launch at 64^3 and 242
-// us at 216^3 against 11.2 and 65) and two-way at worst for packed rows (an odd
-// number of 16-byte units apart), whatever the stage's radix.
+// us at 216^3 against 11.2 and 65), whatever the stage's radix.  Packed rows lie
+// nx + 2 values apart, so theirs conflict gcd(nx + 2, 16)-fold: two-way where
+// nx is a multiple of 4, four-way at nx = 90 or 210, eight-way at 54, 70 or 150,
+// sixteen-way at 14, 30 or 126 (reciprocal space of 20 steps of a few atoms: 1.49
+// ms on 128^3, 2.25 on 126^3; 3.28 and 3.26 with consecutive threads along a row).
 template <int R, bool DIF, bool INV>
 __device__ __forceinline__ void fft_stage(float2 *buf, int nlines, FastDiv by_lines, int lstride,
                                           int estride, int n, int m, FastDiv fmr, const float2 *tw) {
@@ -1324,7 +1327,6 @@ void fill_axis_divisors(FftAxis &a) {
     a.dit_mr[s] = make_fastdiv((unsigned)tail);
     tail *= a.radix[s];
   }
-  a.by_n = make_fastdiv((unsigned)a.n);
   a.by_nxc = make_fastdiv((unsigned)(a.n / 2 + 1));
   a.by_nxcp = make_fastdiv((unsigned)((a.n / 2 + 2) & ~1));
   a.by_ngrp = make_fastdiv((unsigned)((a.n / 2 + 1) / 2 + 1));

@@ -54,7 +54,6 @@ struct FftAxis {
   // decimation-in-frequency (n / radix[0..s]) and the decimation-in-time
   // (radix[s+1..]) passes
   FastDiv dif_mr[8], dit_mr[8];
-  FastDiv by_n;      // x / n
   FastDiv by_nxc;    // x / (n/2 + 1)
   FastDiv by_nxcp;   // x / the even pitch of n/2 + 1
   FastDiv by_ngrp;   // x / ((n/2 + 1)/2 + 1): the real-to-complex split groups
