@@ -13,9 +13,10 @@
 // lanes at once.  Tiles with exclusions (and a cluster's tile with itself) do
 // not go through the queue.  Bound by instruction issue: with the queue, the
 // tiles read 32 at a time and padding slots far away instead of tested, the
-// kernel takes 81 us a launch on 24,000 atoms (98.6 before, 40 steps 6.76 ->
-// 6.41 ms) and 1.69 ms on 998,000 (2.15 before the pair function's and these
-// changes, 20 steps 62.6 -> 58.9 ms).
+// kernel takes 81 us a launch on 24,000 atoms with four blocks an SM, 85 with the
+// three it has there now (98.6 before, 40 steps 6.76 -> 6.41 ms), and 1.69 ms on
+// 998,000 (2.15 before the pair function's and these changes, 20 steps 62.6 ->
+// 58.9 ms).
 #include "nonbonded.h"
 
 #include <algorithm>
