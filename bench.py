@@ -58,9 +58,9 @@ FLOP_PER_PAIR = 65
 # dram__bytes_write.sum) from one ncu capture of the same kernel on the same
 # workload (the inputs and the fixed-point force buffer stay in L2)
 NB_TRAFFIC = {
-    "chain23k": (2193920, "ncu capture of this kernel on this workload "
+    "chain23k": (2099200, "ncu capture of this kernel on this workload "
                           "(dram__bytes_read.sum + dram__bytes_write.sum)"),
-    "chain23k_npt": (2193920, "ncu capture of this kernel on the same system at constant "
+    "chain23k_npt": (2099200, "ncu capture of this kernel on the same system at constant "
                               "volume (dram__bytes_read.sum + dram__bytes_write.sum)"),
 }
 
