@@ -587,11 +587,8 @@ void ForceManager::calcForce(const float4 *d_xyzq, bool calcEnergy, bool calcVir
   m_VirialValid = calcVirial;
   m_EvalMask = m_ComponentMask;
   if (calcEnergy) APO_CUDA(cudaEventRecord(m_EvFork, s));
-  // the reciprocal space first: in a captured segment the first of the fork's
-  // kernels starts ahead of the others, and behind the direct-space grid the
-  // longer chain waited for it (40 steps of 24,000 atoms 5.90 -> 4.61 ms, at
-  // constant pressure 7.66 -> 6.78, of 12,500 2.49 -> 2.46, of 3,000 1.73 -> 1.65)
-  if (m_ComponentMask & 4) {
+  const auto reciprocal = [&] {
+    if (!(m_ComponentMask & 4)) return;
     APO_CUDA(cudaStreamWaitEvent(m_SPme, m_EvFork, 0));
     if (m_Multi)
       m_PmeMulti.compute(m_Nbl.xyzq_s, m_Nbl.cl_origin, m_Nbl.cl_sys, m_Nbl.counts, m_Force.p,
@@ -601,8 +598,9 @@ void ForceManager::calcForce(const float4 *d_xyzq, bool calcEnergy, bool calcVir
                     m_Precise, m_SPme, virial, m_Nbl.cl_origin);
     APO_CUDA(cudaEventRecord(m_EvPme, m_SPme));
     APO_CUDA(cudaStreamWaitEvent(s, m_EvPme, 0));
-  }
-  if (m_ComponentMask & 2) {
+  };
+  const auto direct = [&] {
+    if (!(m_ComponentMask & 2)) return;
     APO_CUDA(cudaStreamWaitEvent(m_SNb, m_EvFork, 0));
     NbArgs a;
     a.xyzq_s = m_Nbl.xyzq_s;
@@ -657,6 +655,23 @@ void ForceManager::calcForce(const float4 *d_xyzq, bool calcEnergy, bool calcVir
     }
     APO_CUDA(cudaEventRecord(m_EvNb, m_SNb));
     APO_CUDA(cudaStreamWaitEvent(s, m_EvNb, 0));
+  };
+  // In a captured segment the first of the fork's kernels starts ahead of the
+  // others, and behind the direct-space grid the longer chain of the reciprocal
+  // space waited for it (40 steps of 24,000 atoms 5.90 -> 4.61 ms, at constant
+  // pressure 7.66 -> 6.78, of 12,500 2.49 -> 2.46, of 3,000 1.73 -> 1.65).  An
+  // evaluation on its own is enqueued while it runs: there five launches ahead
+  // of the direct space hold it up where it is the longer part, in small systems
+  // (with energies, 3,000 atoms 75.7 -> 74.3 us, precise 102.5 -> 94.8, octet lists
+  // 103.3 -> 95.1; 12,500 octet lists 127.0 -> 112.5, but the tile form 93.8 ->
+  // 102.5, and 24,000 160.9 -> 181.3).
+  const int small = m_NbVariant == kNbTileBatches ? 8192 : 16384;
+  if (clear && m_Stride <= small) {
+    direct();
+    reciprocal();
+  } else {
+    reciprocal();
+    direct();
   }
   // bonded terms proper; the 1-4 pairs and exclusion corrections go with
   // them or, under kComponent14WithDirect, with the direct space
