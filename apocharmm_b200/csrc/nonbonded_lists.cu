@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(kOThreads, 5) nbo_kernel(NbArgs a) {
           const float r2raw = dx * dx + dy * dy + dz * dz;
           const bool in = valid && ivalid && !((e >> (16 + l)) & 1u) && r2raw < st.roff2;
           const float2 cc = sh_vdw[tab_off + ti + ((e >> 8) & 0xffu)];
-          const float fij = pair_force<ENERGY>(st, r2raw, in, qi, pj.w, cc, e_elec, e_vdw);
+          const float fij = pair_force<ENERGY, ENERGY>(st, r2raw, in, qi, pj.w, cc, e_elec, e_vdw);
           if (VIRIAL) {
             const float gx = fij * dx, gy = fij * dy, gz = fij * dz;
             vw[0] -= gx * dx;

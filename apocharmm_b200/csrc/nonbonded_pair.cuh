@@ -119,11 +119,15 @@ __device__ __forceinline__ void retire_warp(int *sched, int lane) {
 // One pair: erfc-Ewald (src/CudaDirectForceKernels.cu:479-489) plus VDW_VFSW
 // (src/CudaDirectForceKernels.cu:263-286).  Returns f with gradient on i =
 // f (x_i - x_j); `in` = inside the cutoff and not excluded, anything else
-// gives 0 (whatever r2 then is).  With ENERGY the two energies of the pair
-// are added to e_el / e_vdw.
-template <bool ENERGY>
-__device__ __forceinline__ float pair_force(const NbSetup &st, float r2, bool in, float qi,
+// gives 0 (whatever r2raw then is).  With ENERGY the two energies of the pair
+// are added to e_el / e_vdw.  SPARSE: the energies' arithmetic before the branch
+// on `in`, at r2 = 1 for pairs that are not; the same numbers.  For the octet
+// lists, whose kernel with energies had lost 3 to 6 % to the minimum below (24,000
+// atoms 147.5 -> 150.4 us, with the virial 176.1 -> 186.4; now 140.3 and 167.9).
+template <bool ENERGY, bool SPARSE = false>
+__device__ __forceinline__ float pair_force(const NbSetup &st, float r2raw, bool in, float qi,
                                             float qj, float2 cc, double &e_el, double &e_vdw) {
+  const float r2 = SPARSE && !in ? 1.f : r2raw;
   const float rinv = rsqrt_approx(r2);  // r2 >= 1e-2 inside the cutoff: never denormal
   const float rr = r2 * rinv;
   const float rinv2 = rinv * rinv;
@@ -136,13 +140,15 @@ __device__ __forceinline__ float pair_force(const NbSetup &st, float r2, bool in
   const float g6 = fminf(rinv3, fmaf(st.k6, rinv3, -st.sw6));
   const float g12 = fminf(rinv6, fmaf(st.k12, rinv6, -st.sw12));
   const float fr_vdw = (cc.x * g6) * rinv3 - (cc.y * g12) * rinv6;
-  if (ENERGY && in) {
+  if (ENERGY && (SPARSE || in)) {
     const bool sw = r2 > st.ron2;
     const float t6 = sw ? rinv3 - st.roffinv3 : rinv3, t12 = sw ? rinv6 - st.roffinv6 : rinv6;
     const float C6 = sw ? 0.f : st.dv6, C12 = sw ? 0.f : st.dv12;
-    e_el += (double)el;
-    e_vdw += (double)((1.f / 12.f) * cc.y * (g12 * t12 + C12) -
-                      (1.f / 6.f) * cc.x * (g6 * t6 + C6));
+    const float ev = (1.f / 12.f) * cc.y * (g12 * t12 + C12) - (1.f / 6.f) * cc.x * (g6 * t6 + C6);
+    if (in) {
+      e_el += (double)el;
+      e_vdw += (double)ev;
+    }
   }
   return in ? (fr_vdw + fr_el) * rinv2 : 0.f;
 }
@@ -195,8 +201,8 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
 // packed arithmetic.  To spend no instruction on signs, nqq holds -q_i q_j
 // ccelec and the second Lennard-Jones coefficient comes negated (-12 c12);
 // the electrostatic part is nqq exp(-kappa^2 r^2) (t P(t) / r + 2 kappa /
-// sqrt(pi)) with t P(t) exp(-kappa^2 r^2) = erfc(kappa r).  Bound by
-// instruction issue: 37 packed operations and 14 others for two pairs, where
+// sqrt(pi)) with t P(t) exp(-kappa^2 r^2) = erfc(kappa r).  Its cost
+// is its instructions: 37 packed operations and 14 others for two pairs, where
 // selecting the switch's constants and masking the distances took about 15
 // more (40 steps of 24,000 atoms 6.97 -> 6.76 ms, 20 steps of 998,000 65.6 ->
 // 62.6).  Returns the two values f with gradient on i = f (x_i - x_j); a half that is not `in` gives 0.
